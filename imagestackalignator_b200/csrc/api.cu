@@ -664,13 +664,13 @@ int run_merge(isa_ctx* c, const uint16_t* raw, size_t raw_pitch, size_t frame_st
             gb.yb1 = std::min(g.Ho, y0 + rows);
             const int nr = gb.yb1 - gb.yb0;
             if (p->fused_accumulate) {
-                ISA_LAUNCH(c, isa_launch_accumulate(gb, cfa, c->frame_in, (int)fin.size(), nullptr, raw_pitch, fp, hp4, c->kparam, p4, 4, white, black,
+                ISA_LAUNCH(c, isa_launch_accumulate(gb, cfa, fin.data(), c->frame_in, (int)fin.size(), raw_pitch, fp, hp4, c->kparam, p4, 4, white, black,
                                                     c->acc, c->wsum, op, 0, st));
             } else {
                 ISA_CK(cudaMemsetAsync((char*)c->acc + (size_t)y0 * op, 0, op * nr, st));
                 ISA_CK(cudaMemsetAsync((char*)c->wsum + (size_t)y0 * op, 0, op * nr, st));
                 for (size_t f = 0; f < fin.size(); f++)
-                    ISA_LAUNCH(c, isa_launch_accumulate(gb, cfa, nullptr, 1, &fin[f], raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc,
+                    ISA_LAUNCH(c, isa_launch_accumulate(gb, cfa, &fin[f], nullptr, 1, raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc,
                                                         c->wsum, op, 1, st));
             }
             float* ob = (float*)((char*)out + (size_t)y0 * out_pitch);
@@ -690,13 +690,13 @@ int run_merge(isa_ctx* c, const uint16_t* raw, size_t raw_pitch, size_t frame_st
         return ISA_OK;
     }
     if (p->fused_accumulate) {
-        ISA_LAUNCH(c, isa_launch_accumulate(g, cfa, c->frame_in, (int)fin.size(), nullptr, raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc, c->wsum,
+        ISA_LAUNCH(c, isa_launch_accumulate(g, cfa, fin.data(), c->frame_in, (int)fin.size(), raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc, c->wsum,
                                      op, 0, st));
     } else {
         ISA_CK(cudaMemsetAsync(c->acc, 0, op * g.Ho, st));
         ISA_CK(cudaMemsetAsync(c->wsum, 0, op * g.Ho, st));
         for (size_t f = 0; f < fin.size(); f++)
-            ISA_LAUNCH(c, isa_launch_accumulate(g, cfa, nullptr, 1, &fin[f], raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc, c->wsum, op, 1,
+            ISA_LAUNCH(c, isa_launch_accumulate(g, cfa, &fin[f], nullptr, 1, raw_pitch, fp, hp4, c->kparam, p4, 4, white, black, c->acc, c->wsum, op, 1,
                                          st));
     }
     ISA_TRY(mark());
@@ -1776,7 +1776,7 @@ int isa_accumulate(const uint16_t* raw, size_t raw_pitch, int W, int H, const in
     float r = std::round(scale);
     g.s_int = (r == scale && r >= 1.f) ? (int)r : 0;
     isa_frame_in f{raw, (const float2*)flow, (const float4*)mask};
-    ISA_CK(isa_launch_accumulate(g, pack_cfa(cfa), nullptr, 1, &f, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, kc, white, black, acc,
+    ISA_CK(isa_launch_accumulate(g, pack_cfa(cfa), &f, nullptr, 1, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, kc, white, black, acc,
                                  wsum, out_pitch, 1, S(stream)));
     return ISA_OK;
 }

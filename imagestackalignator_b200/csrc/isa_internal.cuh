@@ -211,15 +211,16 @@ cudaError_t isa_launch_structure_tensor(const float* img, size_t pitch, int W, i
 cudaError_t isa_launch_kernel_param(const float* st3, size_t st_pitch, int W, int H, float* out, size_t out_pitch, int out_channels,
                                     float Dth, float Dtr, float kDetail, float kDenoise, float kStretch, float kShrink,
                                     cudaStream_t st);
-cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes,
-                                  const isa_frame_in* single, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch,
+// frames: host array of the frames to add, in order; frames_dev: the same list on the device (needed where nframes > 1)
+constexpr int ISA_ACC_MAX_FRAMES = 65;  // isa_ctx_create's limit
+cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, const isa_frame_in* frames_dev, int nframes,
+                                  size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch,
                                   int kparam_channels, const float* white, const float* black, float* acc, float* wsum,
                                   size_t out_pitch, int accumulate_into, cudaStream_t st);
-bool isa_accumulate_x2_supported(unsigned cfa);
-cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, const isa_frame_in* single,
-                                     size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch,
-                                     const float* white, const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into,
-                                     cudaStream_t st);
+bool isa_accumulate_x2_supported(const isa_accum_geom& g, unsigned cfa, int nframes, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch);
+cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, size_t raw_pitch,
+                                     size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch, const float* white,
+                                     const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into, cudaStream_t st);
 cudaError_t isa_launch_apply_weighting(float* img, size_t img_pitch, const float* acc, const float* wsum, size_t pitch, int W, int H,
                                        float thr, cudaStream_t st);
 

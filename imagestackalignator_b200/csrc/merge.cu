@@ -574,32 +574,33 @@ cudaError_t isa_launch_kernel_param(const float* st3, size_t st_pitch, int W, in
     return cudaGetLastError();
 }
 
-cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, const isa_frame_in* single,
-                                  size_t raw_pitch,
-                                  size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch, int kparam_channels,
-                                  const float* white, const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into,
-                                  cudaStream_t st)
+cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, const isa_frame_in* frames_dev, int nframes,
+                                  size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch,
+                                  int kparam_channels, const float* white, const float* black, float* acc, float* wsum, size_t out_pitch,
+                                  int accumulate_into, cudaStream_t st)
 {
-    if (!g.bilinear && g.s_int == 2 && kparam_channels == 4 && isa_accumulate_x2_supported(cfa))
-        return isa_launch_accumulate_x2(g, cfa, frames, nframes, single, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc,
-                                        wsum, out_pitch, accumulate_into, st);
+    if (!g.bilinear && g.s_int == 2 && kparam_channels == 4 && isa_accumulate_x2_supported(g, cfa, nframes, raw_pitch, flow_pitch, mask_pitch))
+        return isa_launch_accumulate_x2(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc, wsum,
+                                        out_pitch, accumulate_into, st);
+    if (nframes > 1 && !frames_dev) return cudaErrorInvalidValue;
     F3 wh, bl;
     for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; bl.v[c] = black[c]; }
-    isa_frame_in one = single ? *single : isa_frame_in{nullptr, nullptr, nullptr};
+    const isa_frame_in one = nframes == 1 ? frames[0] : isa_frame_in{nullptr, nullptr, nullptr};
+    const isa_frame_in* list = nframes == 1 ? nullptr : frames_dev;
     if (g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
     dim3 b(g.bx > 0 ? g.bx : 32, g.by > 0 ? g.by : 8), grd = grid2(g.Wo, g.yb1 - g.yb0, b);
     if (b.x * b.y > 256) return cudaErrorInvalidValue;
     if (kparam_channels == 4 && g.bilinear)
-        k_accumulate<4, true><<<grd, b, 0, st>>>(g, cfa, frames, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
+        k_accumulate<4, true><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
                                                  wsum, out_pitch, accumulate_into);
     else if (kparam_channels == 4)
-        k_accumulate<4, false><<<grd, b, 0, st>>>(g, cfa, frames, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
+        k_accumulate<4, false><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
                                                   wsum, out_pitch, accumulate_into);
     else if (kparam_channels == 3 && g.bilinear)
-        k_accumulate<3, true><<<grd, b, 0, st>>>(g, cfa, frames, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
+        k_accumulate<3, true><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
                                                  wsum, out_pitch, accumulate_into);
     else if (kparam_channels == 3)
-        k_accumulate<3, false><<<grd, b, 0, st>>>(g, cfa, frames, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
+        k_accumulate<3, false><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
                                                   wsum, out_pitch, accumulate_into);
     else
         return cudaErrorInvalidValue;

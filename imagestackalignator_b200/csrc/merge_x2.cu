@@ -12,36 +12,55 @@
 // (X + p) >> 2, so which of the two mask columns a tap reads depends only on
 // X mod 4 (and rows on Y mod 4).
 //
-// Work layout. A CTA of 8 warps covers output columns bx*128 + 4*lane + ph
-// and rows by*32 + 4*warp + rph, so X mod 4 and Y mod 4 are the same for
-// every thread of the CTA: the tap -> mask-quadrant pattern is a template
-// parameter (16 instantiations, chosen per CTA). The parity of (Xs, Ys)
-// still varies from pixel to pixel; it is applied with selects, never with
-// branches:
-//   per tap row, the five weighted taps fold into three cell weights, the
-//   taps -1 and +1 going to one of two cells by the column parity;
-//   the five rows fold into three cell rows the same way by the row parity;
-//   the 3 x 3 cell weights multiply the 3 x 3 samples into the four
-//   relative CFA classes, which map to R, G, B through two bits per frame.
+// Work layout. A warp covers 32 output pixels of one row, four columns apart
+// (x = 128 bx + 4 lane + ph), so X mod 4 and Y mod 4 are the same for the
+// whole warp. A CTA is the four ph of 128-pixel segments of four rows of one
+// Y mod 4: its warps share the source lines they read, and the segments are
+// written in whole lines through shared memory.
+//
+// The taps of a line fall into four groups of one cell and one mask line each,
+// whatever the parity of Xs: that parity only moves the taps -1 and +1 between
+// neighbouring groups, by multiply-adds with a 0 / 1 factor (the FMA pipe has
+// room, the ALU pipe that selects run on does not). So the 5 x 5 weights (13
+// distinct: w(-p) = w(p)) fold to 4 x 4 group weights, and the certainties
+// meet them once per group:
+//   W(cell) = sum over the cell's groups of (group weight) (certainty),
+// with the certainty of the group's relative CFA class in its mask cell.
+// The 3 x 3 cell weights multiply the 3 x 3 samples into the four relative
+// CFA classes, which map to R, G, B through two bits per frame.
 // Per frame and channel: acc_c += (sum w cert raw - black_c sum w cert) /
 // white_c, wsum_c += sum w cert: the reference's per-tap
 // (raw - black_c) / white_c * w * cert summed over the taps of the frame.
-// Pixels whose 3 x 3 block or mask window reaches the crop border take a
-// per-tap path with the reference's clamps.
+// Pixels whose 3 x 3 block, mask window or flow cell reaches a border (and
+// weights so large that their sums could overflow) take a per-tap path with
+// the reference's clamps, out of line.
+//
+// Bound: instruction issue and instruction fetch, about 290 instructions per
+// pixel and frame at an IPC near 2.7. Code size decides as much as the count:
+// the frame loop is one body per Y mod 4 (uniform in a CTA, and the rows of a
+// 32-row band run one Y mod 4 after another) with a 35-instruction section
+// per X mod 4. One body per (X mod 4, Y mod 4) pair inside a CTA took 157 ms
+// at 20 x 6016x4000 (the instruction cache thrashes), the same bodies with
+// CTA-uniform X mod 4 23.3 ms (the sixteen interleaved CTAs re-read each line
+// from L2), four pixels per thread 36 ms (a 16 KB body), group weights in a
+// shared-memory table 28-34 ms (no L1 left for the frames). This form: 23.4 ms,
+// from 25.4 ms for per-tap selects; one 4096x3072 frame by itself 0.54 ms, from
+// 0.87 ms. CTAs of 256 threads take 22.5 ms, but where bursts are merged side by
+// side on several streams small CTAs refill every slot they free and keep the
+// other streams' larger CTAs waiting (six bursts of 6 x 1024x768 on three
+// streams: 7.78 ms with 256 threads, 7.48 ms with 512).
 #include "isa_internal.cuh"
 
 namespace {
+
+constexpr int X2_W = 128, X2_ROWS = 4;  // row segment of a CTA's 128-thread part, rows (of one y mod 4) per CTA
+constexpr int X2_NT = X2_W * X2_ROWS, X2_CTAS = 2;  // threads of a CTA, CTAs per SM
 
 struct C3 { float v[3]; };
 
 // Bayer description: green where (row parity ^ column parity) == g0, red on
 // rows with parity ry.
 struct Bayer { int g0, ry; };
-
-// Mask column (0/1, relative to (X - 2) >> 2) of tap p for X mod 4 == M.
-__host__ __device__ constexpr int quad_of(int M, int p) { return ((M + p + 4) >> 2) - ((M + 2) >> 2); }
-
-__device__ __forceinline__ float comp(const float4& m, int ch) { return ch == 0 ? m.x : (ch == 1 ? m.y : m.z); }
 
 __device__ __forceinline__ float4 sanitize(float4 m)
 {
@@ -63,40 +82,55 @@ __device__ __forceinline__ void class_certs(const float4& m, bool hG, bool fr, f
     c[3] = hG ? m.y : rb1;
 }
 
-// One tap row: weights w[0..4] (taps -2..2), certainties cc[mask column][cell
-// column parity] of the row, column parity PX of Xs -> cell weights R0..R2.
-template <int XM>
-__device__ __forceinline__ void row_cells(float w0, float w1, float w2, float w3, float w4, const float (&cc)[2][2], bool PX, float& R0, float& R1,
-                                          float& R2)
+// The five taps of a line (-2 .. 2) into the four groups of X mod 4 == M (rows alike). P = 1, nP = 0 where the shifted
+// position is odd, else P = 0, nP = 1. (Even: taps -2 -1 | 0 +1 | +2 share cells; odd: -2 | -1 0 | +1 +2.)
+template <int M>
+__device__ __forceinline__ void fold(float w0, float w1, float w2, float w3, float w4, float P, float nP, float (&g)[4])
 {
-    constexpr int d0 = quad_of(XM, -2), d1 = quad_of(XM, -1), d2 = quad_of(XM, 0), d3 = quad_of(XM, 1), d4 = quad_of(XM, 2);
-    const float t0 = w0 * cc[d0][0];
-    const float t2 = w2 * cc[d2][1];
-    const float t4 = w4 * cc[d4][0];
-    const float tm = w1 * (PX ? cc[d1][1] : cc[d1][0]);  // tap -1: cell PX
-    const float tp = w3 * (PX ? cc[d3][0] : cc[d3][1]);  // tap +1: cell 1 + PX
-    R0 = PX ? t0 : t0 + tm;
-    R1 = t2 + (PX ? tm : tp);
-    R2 = PX ? t4 + tp : t4;
+    if constexpr (M == 0) {         // mask lines: -2 -1 | 0 +1 +2
+        g[0] = fmaf(nP, w1, w0); g[1] = P * w1; g[2] = fmaf(nP, w3, w2); g[3] = fmaf(P, w3, w4);
+    } else if constexpr (M == 1) {  // -2 | -1 0 +1 +2
+        g[0] = w0; g[1] = nP * w1; g[2] = fmaf(nP, w3, fmaf(P, w1, w2)); g[3] = fmaf(P, w3, w4);
+    } else if constexpr (M == 2) {  // -2 -1 0 +1 | +2
+        g[0] = fmaf(nP, w1, w0); g[1] = fmaf(nP, w3, fmaf(P, w1, w2)); g[2] = P * w3; g[3] = w4;
+    } else {                        // -2 -1 0 | +1 +2
+        g[0] = fmaf(nP, w1, w0); g[1] = fmaf(P, w1, w2); g[2] = nP * w3; g[3] = fmaf(P, w3, w4);
+    }
 }
 
-// Row certainties for a tap row in mask row DR whose cell row has parity rp.
-template <int DR>
-__device__ __forceinline__ void row_certs(const float (&cq)[2][2][4], bool rp, float (&cc)[2][2])
+// Cell and mask line of group g for X mod 4 == M.
+__host__ __device__ constexpr int cell_of(int M, int g) { return g == 0 ? 0 : (g == 3 ? 2 : (g == 1 ? (M == 1 ? 0 : 1) : (M == 2 ? 2 : 1))); }
+__host__ __device__ constexpr int mline_of(int M, int g) { return g == 0 ? 0 : (g == 3 ? 1 : (g == 1 ? (M == 1 ? 1 : 0) : (M == 2 ? 0 : 1))); }
+
+// Tap weights and certainties cq[mask row][mask column][class] -> cell weights: columns to groups, then rows, then the
+// groups' certainties.
+template <int XM, int YM>
+__device__ __forceinline__ void cells(const float (&w)[5][5], float Q, float nQ, float P, float nP, const float (&cq)[2][2][4], float (&Wc)[3][3])
 {
+    bool set[3][3] = {};
+    float G[5][4];
 #pragma unroll
-    for (int dc = 0; dc < 2; dc++)
+    for (int r = 0; r < 5; r++) fold<XM>(w[r][0], w[r][1], w[r][2], w[r][3], w[r][4], P, nP, G[r]);
 #pragma unroll
-        for (int cp = 0; cp < 2; cp++) cc[dc][cp] = rp ? cq[DR][dc][2 + cp] : cq[DR][dc][cp];
+    for (int c = 0; c < 4; c++) {
+        float u[4];
+        fold<YM>(G[0][c], G[1][c], G[2][c], G[3][c], G[4][c], Q, nQ, u);
+        const int i = cell_of(XM, c);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int j = cell_of(YM, r);
+            const float k = cq[mline_of(YM, r)][mline_of(XM, c)][(j & 1) * 2 + (i & 1)];
+            Wc[j][i] = set[j][i] ? fmaf(u[r], k, Wc[j][i]) : u[r] * k;
+            set[j][i] = true;
+        }
+    }
 }
 
 struct X2Args {
     isa_accum_geom g;
     unsigned cfa;
     Bayer bayer;
-    const isa_frame_in* frames;
     int nframes;
-    isa_frame_in single;
     size_t raw_pitch, flow_pitch, mask_pitch;
     const float4* kparam;
     size_t kp_pitch;
@@ -105,193 +139,258 @@ struct X2Args {
     float* wsum;
     size_t out_pitch;
     int accumulate_into;
+    isa_frame_in frames[ISA_ACC_MAX_FRAMES];
 };
 
-template <int XM, int YM, bool SANE>
-__device__ __forceinline__ void pixel_x2(const X2Args& A, int x, int y)
+// What a frame without flow or mask reads, at offset 0.
+__device__ const float4 g_zero_flow = {0.f, 0.f, 0.f, 0.f};
+__device__ const float4 g_unit_mask[2] = {{1.f, 1.f, 1.f, 1.f}, {1.f, 1.f, 1.f, 1.f}};
+
+struct Sums { float a[3], w[3]; };
+
+// Sample position of output pixel (x, y): texel and sub-pixel part.
+struct Position { int ib, jb; float ax, by; };
+
+__device__ __forceinline__ Position position(const isa_accum_geom& g, int x, int y)
 {
-    const isa_accum_geom& g = A.g;
-    float* ap = isa::row_ptr(A.acc, A.out_pitch, y) + 3 * x;
-    float* wp = isa::row_ptr(A.wsum, A.out_pitch, y) + 3 * x;
-    if (x < 1 || y < 1 || x >= g.Wo - 1 || y >= g.Ho - 1) {
-        if (!A.accumulate_into) { ap[0] = ap[1] = ap[2] = 0.f; wp[0] = wp[1] = wp[2] = 0.f; }
-        return;
-    }
-    float a[3] = {0.f, 0.f, 0.f}, ws[3] = {0.f, 0.f, 0.f};
-    if (A.accumulate_into) {
-        a[0] = ap[0]; a[1] = ap[1]; a[2] = ap[2];
-        ws[0] = wp[0]; ws[1] = wp[1]; ws[2] = wp[2];
-    }
-    const int X = x + g.ox, Y = y + g.oy;
     const float xb = ((float)x + 0.5f + (float)g.ox) / 2.0f - 0.5f;
     const float yb = ((float)y + 0.5f + (float)g.oy) / 2.0f - 0.5f;
     const float fxb = floorf(xb), fyb = floorf(yb);
-    const int ib = (int)fxb, jb = (int)fyb;
-    const float ax = xb - fxb, by = yb - fyb;
-    // kernel parameters: bilinear, clamp addressing
-    float k0p, k1p, k2p;
-    {
-        const int i0 = isa::clampi(ib, 0, g.W - 1), i1 = isa::clampi(ib + 1, 0, g.W - 1);
-        const int j0 = isa::clampi(jb, 0, g.H - 1), j1 = isa::clampi(jb + 1, 0, g.H - 1);
-        const float4 p00 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j0) + i0), p10 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j0) + i1);
-        const float4 p01 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j1) + i0), p11 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j1) + i1);
-        k0p = isa::lerp2(p00.x, p10.x, p01.x, p11.x, ax, by);
-        k1p = isa::lerp2(p00.y, p10.y, p01.y, p11.y, ax, by);
-        k2p = isa::lerp2(p00.z, p10.z, p01.z, p11.z, ax, by);
-    }
-    float w[5][5];
+    return {(int)fxb, (int)fyb, xb - fxb, yb - fyb};
+}
+
+// Kernel parameters: bilinear, clamp addressing.
+__device__ __forceinline__ void kernel_params(const X2Args& A, const Position& p, float& k0, float& k1, float& k2)
+{
+    const isa_accum_geom& g = A.g;
+    const int i0 = isa::clampi(p.ib, 0, g.W - 1), i1 = isa::clampi(p.ib + 1, 0, g.W - 1);
+    const int j0 = isa::clampi(p.jb, 0, g.H - 1), j1 = isa::clampi(p.jb + 1, 0, g.H - 1);
+    const float4 p00 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j0) + i0), p10 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j0) + i1);
+    const float4 p01 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j1) + i0), p11 = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, j1) + i1);
+    k0 = isa::lerp2(p00.x, p10.x, p01.x, p11.x, p.ax, p.by);
+    k1 = isa::lerp2(p00.y, p10.y, p01.y, p11.y, p.ax, p.by);
+    k2 = isa::lerp2(p00.z, p10.z, p01.z, p11.z, p.ax, p.by);
+}
+
+// The 13 distinct tap weights, w(-p) = w(p), from the kernel parameters; returns the largest.
+__device__ __forceinline__ float tap_weights(float k0, float k1, float k2, float (&w)[5][5])
+{
+    float wmax = 1.f;
 #pragma unroll
-    for (int py = -2; py <= 2; py++)
+    for (int py = 0; py <= 2; py++)
 #pragma unroll
         for (int px = -2; px <= 2; px++) {
-            float q = px * px * k0p + 2 * px * py * k2p + py * py * k1p;
-            float vv = expf(-0.5f * q);
-            if (!isfinite(vv)) vv = px * py == 0 ? 1.f : 0.f;
-            w[py + 2][px + 2] = vv;
+            if (py == 0 && px < 0) continue;
+            float v = 1.f;
+            if (py != 0 || px != 0) {
+                const float q = px * px * k0 + 2 * px * py * k2 + py * py * k1;
+                v = expf(-0.5f * q);
+                if (!isfinite(v)) v = px * py == 0 ? 1.f : 0.f;
+                wmax = fmaxf(wmax, v);
+            }
+            w[2 + py][2 + px] = w[2 - py][2 - px] = v;
         }
-    // flow: bilinear, mirror addressing (same position for every frame)
-    const int fi0 = isa::mirror(ib, g.W), fi1 = isa::mirror(ib + 1, g.W);
-    const size_t fr0 = (size_t)isa::mirror(jb, g.H) * A.flow_pitch, fr1 = (size_t)isa::mirror(jb + 1, g.H) * A.flow_pitch;
-    // interior: the unshifted taps' mask cells are (X - 2) >> 2 + {0, 1}, rows alike,
-    // and the shifted 3 x 3 block [k0, k0 + 2] x [j0, j0 + 2] lies inside the crop:
-    // k0 = (X + sx - 2) >> 1 in [cx0, cx1 - 2]  <=>  sx in [2 cx0 + 2 - X, 2 cx1 - 1 - X]
-    const bool mask_interior = ((X - 2) >> 1) >= g.cx0 && ((X + 2) >> 1) <= g.cx1 && ((Y - 2) >> 1) >= g.cy0 && ((Y + 2) >> 1) <= g.cy1;
-    const int sxlo = mask_interior ? 2 * g.cx0 + 2 - X : (1 << 29), sylo = 2 * g.cy0 + 2 - Y;
-    const unsigned sxspan = mask_interior ? (unsigned)(2 * g.cx1 - 1 - X - sxlo) : 0u, syspan = (unsigned)(2 * g.cy1 - 1 - Y - sylo);
-    const int ux0 = (X - 2) >> 2, uy0 = (Y - 2) >> 2;
-    const size_t moff = (size_t)uy0 * A.mask_pitch + (size_t)ux0 * sizeof(float4);
-    for (int f = 0; f < A.nframes; f++) {
-        const isa_frame_in fr = A.frames ? A.frames[f] : A.single;
-        int sx = 0, sy = 0;
-        if (fr.flow) {
-            const char* fb = (const char*)fr.flow;
-            const float2 p00 = __ldg((const float2*)(fb + fr0) + fi0), p10 = __ldg((const float2*)(fb + fr0) + fi1);
-            const float2 p01 = __ldg((const float2*)(fb + fr1) + fi0), p11 = __ldg((const float2*)(fb + fr1) + fi1);
-            sx = (int)roundf(isa::lerp2(p00.x, p10.x, p01.x, p11.x, ax, by) * 2.0f);
-            sy = (int)roundf(isa::lerp2(p00.y, p10.y, p01.y, p11.y, ax, by) * 2.0f);
+    return wmax;
+}
+
+// One frame's sums of a pixel tap by tap, with the crop clamps and mirrored flow of the reference.
+__device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
+{
+    const isa_accum_geom& g = A.g;
+    const isa_frame_in fr = A.frames[f];
+    const Position p = position(g, x, y);
+    const int X = x + g.ox, Y = y + g.oy;
+    float k0, k1, k2, w[5][5];
+    kernel_params(A, p, k0, k1, k2);
+    tap_weights(k0, k1, k2, w);
+    Sums s = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    int sx = 0, sy = 0;
+    if (fr.flow) {
+        const int i0 = isa::mirror(p.ib, g.W), i1 = isa::mirror(p.ib + 1, g.W);
+        const float2* r0 = isa::row_ptr(fr.flow, A.flow_pitch, isa::mirror(p.jb, g.H));
+        const float2* r1 = isa::row_ptr(fr.flow, A.flow_pitch, isa::mirror(p.jb + 1, g.H));
+        const float2 p00 = __ldg(r0 + i0), p10 = __ldg(r0 + i1), p01 = __ldg(r1 + i0), p11 = __ldg(r1 + i1);
+        sx = (int)roundf(isa::lerp2(p00.x, p10.x, p01.x, p11.x, p.ax, p.by) * 2.0f);
+        sy = (int)roundf(isa::lerp2(p00.y, p10.y, p01.y, p11.y, p.ax, p.by) * 2.0f);
+    }
+    int qx[5], ux[5];
+#pragma unroll
+    for (int d = 0; d < 5; d++) {
+        qx[d] = isa::clampi((X + sx + d - 2) >> 1, g.cx0, g.cx1);
+        ux[d] = (isa::clampi((X + d - 2) >> 1, g.cx0, g.cx1) >> 1) * 4;
+    }
+#pragma unroll
+    for (int py = -2; py <= 2; py++) {
+        const int qy = isa::clampi((Y + sy + py) >> 1, g.cy0, g.cy1);
+        const int uy = isa::clampi((Y + py) >> 1, g.cy0, g.cy1) >> 1;
+        const uint16_t* rr = isa::row_ptr(fr.raw, A.raw_pitch, qy);
+        const float* mr = fr.mask ? (const float*)isa::row_ptr(fr.mask, A.mask_pitch, uy) : nullptr;
+#pragma unroll
+        for (int d = 0; d < 5; d++) {
+            const int c = isa::cfa_at(A.cfa, qx[d], qy);
+            float cert = 1.f;
+            if (mr) {
+                cert = __ldg(mr + ux[d] + c);
+                if (!isfinite(cert)) cert = 0.f;
+            }
+            const float wc = __fmul_rn(w[py + 2][d], cert);
+            const float raw = (float)__ldg(rr + qx[d]);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (k == c) { s.w[k] = __fadd_rn(s.w[k], wc); s.a[k] = __fmaf_rn(wc, raw, s.a[k]); }
         }
-        const int Xs = X + sx, Ys = Y + sy;
+    }
+    return s;
+}
+
+// Frames f0, f0 + 1, ... of output pixel (x, y), y mod 4 (with the origin) == YM, up to the first whose 3 x 3 block
+// reaches a border (returned); w: the tap weights; interior: neither the unshifted taps' mask cells nor the flow's
+// texels reach a border.
+template <int YM, bool SANE>
+__device__ __forceinline__ int frames_x2(const X2Args& A, int f0, int x, int y, const float (&w)[5][5], bool interior, float (&a)[3], float (&ws)[3])
+{
+    const isa_accum_geom& g = A.g;
+    const int X = x + g.ox, Y = y + g.oy, XM = X & 3;
+    const Position p = position(g, x, y);
+    // bilinear weights of the flow sample (never zero at scale 2), combined in lerp2's order and rounding
+    const float f00 = (1.f - p.ax) * (1.f - p.by), f10 = p.ax * (1.f - p.by), f01 = (1.f - p.ax) * p.by, f11 = p.ax * p.by;
+    const unsigned foff = (unsigned)isa::clampi(p.jb, 0, g.H - 2) * (unsigned)A.flow_pitch + (unsigned)isa::clampi(p.ib, 0, g.W - 2) * 8u;
+    const unsigned moff = (unsigned)isa::clampi((Y - 2) >> 2, 0, g.H / 2 - 2) * (unsigned)A.mask_pitch + (unsigned)isa::clampi((X - 2) >> 2, 0, g.W / 2 - 2) * 16u;
+    // the shifted 3 x 3 block lies inside the crop: k0 in [cx0, cx1 - 2], j0 in [cy0, cy1 - 2]
+    const unsigned kspan = (unsigned)(g.cx1 - 2 - g.cx0), jspan = (unsigned)(g.cy1 - 2 - g.cy0);
+    int f = f0;
+#pragma unroll 1
+    for (; f < A.nframes; f++) {
+        const char* fl = (const char*)A.frames[f].flow;
+        const char* fb = fl ? fl : (const char*)&g_zero_flow;
+        const char* fb1 = fb + (fl ? A.flow_pitch : 0);
+        const unsigned fo = fl ? foff : 0u;
+        const float2 p00 = __ldg((const float2*)(fb + fo)), p10 = __ldg((const float2*)(fb + fo) + 1);
+        const float2 p01 = __ldg((const float2*)(fb1 + fo)), p11 = __ldg((const float2*)(fb1 + fo) + 1);
+        const float flx = __fmaf_rn(f11, p11.x, __fmaf_rn(f01, p01.x, __fmaf_rn(f10, p10.x, __fmul_rn(f00, p00.x))));
+        const float fly = __fmaf_rn(f11, p11.y, __fmaf_rn(f01, p01.y, __fmaf_rn(f10, p10.y, __fmul_rn(f00, p00.y))));
+        const int Xs = X + (int)roundf(flx * 2.0f), Ys = Y + (int)roundf(fly * 2.0f);
         const int k0 = (Xs - 2) >> 1, j0 = (Ys - 2) >> 1;
-        float Ac[3] = {0.f, 0.f, 0.f}, Wc[3] = {0.f, 0.f, 0.f};
-        if ((unsigned)(sx - sxlo) <= sxspan && (unsigned)(sy - sylo) <= syspan) {
-            float v[3][3];
+        if (!(interior && (unsigned)(k0 - g.cx0) <= kspan && (unsigned)(j0 - g.cy0) <= jspan)) {
+            break;
+        }
+        const unsigned ro = (unsigned)j0 * (unsigned)A.raw_pitch + 2u * (unsigned)k0;
+        float v[3][3];
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const uint16_t* rr = isa::row_ptr(fr.raw, A.raw_pitch, j0 + j) + k0;
-                v[j][0] = (float)__ldg(rr);
-                v[j][1] = (float)__ldg(rr + 1);
-                v[j][2] = (float)__ldg(rr + 2);
-            }
-            const bool fx = k0 & 1, fy = j0 & 1;
-            const bool hG = (int)(fx ^ fy) == A.bayer.g0, frr = (int)fy == A.bayer.ry;
-            float cq[2][2][4];
-            if (fr.mask) {
-                const float4* m0 = (const float4*)((const char*)fr.mask + moff);
-                const float4* m1 = (const float4*)((const char*)fr.mask + moff + A.mask_pitch);
-                float4 M00 = __ldg(m0), M01 = __ldg(m0 + 1), M10 = __ldg(m1), M11 = __ldg(m1 + 1);
-                if (!SANE) { M00 = sanitize(M00); M01 = sanitize(M01); M10 = sanitize(M10); M11 = sanitize(M11); }
-                class_certs(M00, hG, frr, cq[0][0]);
-                class_certs(M01, hG, frr, cq[0][1]);
-                class_certs(M10, hG, frr, cq[1][0]);
-                class_certs(M11, hG, frr, cq[1][1]);
-            } else {
+        for (int j = 0; j < 3; j++) {
+            const uint16_t* rr = (const uint16_t*)((const char*)A.frames[f].raw + j * A.raw_pitch + ro);
+            v[j][0] = (float)__ldg(rr);
+            v[j][1] = (float)__ldg(rr + 1);
+            v[j][2] = (float)__ldg(rr + 2);
+        }
+        const char* mk = (const char*)A.frames[f].mask;
+        const char* mb = mk ? mk : (const char*)g_unit_mask;
+        const char* mb1 = mb + (mk ? A.mask_pitch : 0);
+        const unsigned mo = mk ? moff : 0u;
+        float4 M00 = __ldg((const float4*)(mb + mo)), M01 = __ldg((const float4*)(mb + mo) + 1);
+        float4 M10 = __ldg((const float4*)(mb1 + mo)), M11 = __ldg((const float4*)(mb1 + mo) + 1);
+        const bool fx = k0 & 1, fy = j0 & 1;
+        const bool hG = (int)(fx ^ fy) == A.bayer.g0, frr = (int)fy == A.bayer.ry;
+        float cq[2][2][4];
+        if (!SANE) { M00 = sanitize(M00); M01 = sanitize(M01); M10 = sanitize(M10); M11 = sanitize(M11); }
+        class_certs(M00, hG, frr, cq[0][0]);
+        class_certs(M01, hG, frr, cq[0][1]);
+        class_certs(M10, hG, frr, cq[1][0]);
+        class_certs(M11, hG, frr, cq[1][1]);
+        const float P = (Xs & 1) ? 1.f : 0.f, nP = 1.f - P, Q = (Ys & 1) ? 1.f : 0.f, nQ = 1.f - Q;
+        float Wc[3][3];
+        // the same for the whole warp
+        if (XM == 0) cells<0, YM>(w, Q, nQ, P, nP, cq, Wc);
+        else if (XM == 1) cells<1, YM>(w, Q, nQ, P, nP, cq, Wc);
+        else if (XM == 2) cells<2, YM>(w, Q, nQ, P, nP, cq, Wc);
+        else cells<3, YM>(w, Q, nQ, P, nP, cq, Wc);
+        // relative classes
+        const float A0 = __fmaf_rn(Wc[2][2], v[2][2], __fmaf_rn(Wc[2][0], v[2][0], __fmaf_rn(Wc[0][2], v[0][2], __fmul_rn(Wc[0][0], v[0][0]))));
+        const float A1 = __fmaf_rn(Wc[2][1], v[2][1], __fmul_rn(Wc[0][1], v[0][1]));
+        const float A2 = __fmaf_rn(Wc[1][2], v[1][2], __fmul_rn(Wc[1][0], v[1][0]));
+        const float A3 = __fmul_rn(Wc[1][1], v[1][1]);
+        const float W0 = __fadd_rn(__fadd_rn(Wc[0][0], Wc[0][2]), __fadd_rn(Wc[2][0], Wc[2][2]));
+        const float W1 = __fadd_rn(Wc[0][1], Wc[2][1]);
+        const float W2 = __fadd_rn(Wc[1][0], Wc[1][2]);
+        const float W3 = Wc[1][1];
+        // relative classes -> R, G, B
+        const float NA0 = hG ? A1 : A0, NA1 = hG ? A2 : A3, NW0 = hG ? W1 : W0, NW1 = hG ? W2 : W3;
+        const float ga = __fadd_rn(hG ? A0 : A1, hG ? A3 : A2), gw = __fadd_rn(hG ? W0 : W1, hG ? W3 : W2);
+        const float ra = frr ? NA0 : NA1, ba = frr ? NA1 : NA0, rw = frr ? NW0 : NW1, bw = frr ? NW1 : NW0;
+        a[0] = __fmaf_rn(__fmaf_rn(-A.black.v[0], rw, ra), A.rwhite.v[0], a[0]);
+        a[1] = __fmaf_rn(__fmaf_rn(-A.black.v[1], gw, ga), A.rwhite.v[1], a[1]);
+        a[2] = __fmaf_rn(__fmaf_rn(-A.black.v[2], bw, ba), A.rwhite.v[2], a[2]);
+        ws[0] = __fadd_rn(ws[0], rw);
+        ws[1] = __fadd_rn(ws[1], gw);
+        ws[2] = __fadd_rn(ws[2], bw);
+    }
+    return f;
+}
+
+template <bool SANE>
+__global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_constant__ X2Args A)
+{
+    __shared__ float so[X2_ROWS][2][3 * X2_W];
+    const isa_accum_geom& g = A.g;
+    const int tid = threadIdx.x % X2_W, lane = tid & 31, ph = tid >> 5, part = threadIdx.x / X2_W;
+    // blocks in bands of 32 rows, eight CTA rows each, two per y mod 4: the CTAs of an SM run the same code
+    const int nbx = (g.Wo + X2_W - 1) / X2_W;
+    const int row = blockIdx.x / nbx, r = row & 7;
+    const int x0 = (blockIdx.x - row * nbx) * X2_W, y = g.yb0 + 4 * (row & ~7) + 4 * (4 * (r & 1) + part) + (r >> 1);
+    const bool yin = y < g.yb1;
+    const int nx = yin ? 3 * min(X2_W, g.Wo - x0) : 0;
+    float* arow = isa::row_ptr(A.acc, A.out_pitch, y) + 3 * x0;
+    float* wrow = isa::row_ptr(A.wsum, A.out_pitch, y) + 3 * x0;
+    if (A.accumulate_into) {
 #pragma unroll
-                for (int i = 0; i < 16; i++) (&cq[0][0][0])[i] = 1.f;
-            }
-            const bool PX = Xs & 1, PY = Ys & 1;
-            // tap rows -> cell weights per row (rows -1 and +1 have cell-row parity PY and !PY)
-            float Rm2[3], Rm1[3], R0[3], Rp1[3], Rp2[3];
-            {
-                float cc[2][2];
-                row_certs<quad_of(YM, -2)>(cq, false, cc);
-                row_cells<XM>(w[0][0], w[0][1], w[0][2], w[0][3], w[0][4], cc, PX, Rm2[0], Rm2[1], Rm2[2]);
-                row_certs<quad_of(YM, -1)>(cq, PY, cc);
-                row_cells<XM>(w[1][0], w[1][1], w[1][2], w[1][3], w[1][4], cc, PX, Rm1[0], Rm1[1], Rm1[2]);
-                row_certs<quad_of(YM, 0)>(cq, true, cc);
-                row_cells<XM>(w[2][0], w[2][1], w[2][2], w[2][3], w[2][4], cc, PX, R0[0], R0[1], R0[2]);
-                row_certs<quad_of(YM, 1)>(cq, !PY, cc);
-                row_cells<XM>(w[3][0], w[3][1], w[3][2], w[3][3], w[3][4], cc, PX, Rp1[0], Rp1[1], Rp1[2]);
-                row_certs<quad_of(YM, 2)>(cq, false, cc);
-                row_cells<XM>(w[4][0], w[4][1], w[4][2], w[4][3], w[4][4], cc, PX, Rp2[0], Rp2[1], Rp2[2]);
-            }
-            float Wcell[3][3];
+        for (int k = 0; k < 3; k++) {
+            const int i = tid + k * X2_W;
+            if (i < nx) { so[part][0][i] = arow[i]; so[part][1][i] = wrow[i]; }
+        }
+        __syncthreads();
+    }
+    const int lx = 4 * lane + ph, x = x0 + lx;
+    if (yin && x < g.Wo) {
+        float a[3] = {0.f, 0.f, 0.f}, ws[3] = {0.f, 0.f, 0.f};
+        if (A.accumulate_into) {
 #pragma unroll
-            for (int i = 0; i < 3; i++) {
-                Wcell[0][i] = PY ? Rm2[i] : Rm2[i] + Rm1[i];
-                Wcell[1][i] = R0[i] + (PY ? Rm1[i] : Rp1[i]);
-                Wcell[2][i] = PY ? Rp2[i] + Rp1[i] : Rp2[i];
-            }
-            // relative classes
-            const float A0 = Wcell[0][0] * v[0][0] + Wcell[0][2] * v[0][2] + Wcell[2][0] * v[2][0] + Wcell[2][2] * v[2][2];
-            const float A1 = Wcell[0][1] * v[0][1] + Wcell[2][1] * v[2][1];
-            const float A2 = Wcell[1][0] * v[1][0] + Wcell[1][2] * v[1][2];
-            const float A3 = Wcell[1][1] * v[1][1];
-            const float W0 = Wcell[0][0] + Wcell[0][2] + Wcell[2][0] + Wcell[2][2];
-            const float W1 = Wcell[0][1] + Wcell[2][1];
-            const float W2 = Wcell[1][0] + Wcell[1][2];
-            const float W3 = Wcell[1][1];
-            // relative classes -> R, G, B
-            const float NA0 = hG ? A1 : A0, NA1 = hG ? A2 : A3, NW0 = hG ? W1 : W0, NW1 = hG ? W2 : W3;
-            Ac[1] = hG ? A0 + A3 : A1 + A2;
-            Wc[1] = hG ? W0 + W3 : W1 + W2;
-            Ac[0] = frr ? NA0 : NA1;
-            Ac[2] = frr ? NA1 : NA0;
-            Wc[0] = frr ? NW0 : NW1;
-            Wc[2] = frr ? NW1 : NW0;
-        } else {
-            // border: per-tap reference arithmetic with the crop clamps
-#pragma unroll 1
-            for (int py = -2; py <= 2; py++) {
-                const int qy = isa::clampi((Ys + py) >> 1, g.cy0, g.cy1);
-                const int uy = isa::clampi((Y + py) >> 1, g.cy0, g.cy1) >> 1;
-                const uint16_t* rr = isa::row_ptr(fr.raw, A.raw_pitch, qy);
-                const float4* mr = fr.mask ? isa::row_ptr(fr.mask, A.mask_pitch, uy) : nullptr;
-#pragma unroll 1
-                for (int px = -2; px <= 2; px++) {
-                    const int qx = isa::clampi((Xs + px) >> 1, g.cx0, g.cx1);
-                    const int ux = isa::clampi((X + px) >> 1, g.cx0, g.cx1) >> 1;
-                    const int c = isa::cfa_at(A.cfa, qx, qy);
-                    float cert = 1.f;
-                    if (mr) {
-                        cert = comp(__ldg(mr + ux), c);
-                        if (!isfinite(cert)) cert = 0.f;
-                    }
-                    // the weight is recomputed here: indexing w[][] with loop
-                    // counters would move the array out of registers
-                    float wv = expf(-0.5f * (px * px * k0p + 2 * px * py * k2p + py * py * k1p));
-                    if (!isfinite(wv)) wv = px * py == 0 ? 1.f : 0.f;
-                    const float wc = wv * cert;
-                    const float raw = (float)__ldg(rr + qx);
+            for (int c = 0; c < 3; c++) { a[c] = so[part][0][3 * lx + c]; ws[c] = so[part][1][3 * lx + c]; }
+        }
+        if (x >= 1 && y >= 1 && x < g.Wo - 1 && y < g.Ho - 1) {
+            const int X = x + g.ox, Y = y + g.oy;
+            const Position p = position(g, x, y);
+            float k0, k1, k2, w[5][5];
+            kernel_params(A, p, k0, k1, k2);
+            const float wmax = tap_weights(k0, k1, k2, w);
+            // the unshifted taps' mask cells are (X - 2) >> 2 + {0, 1} inside the crop, rows alike, the crop holds a 3 x 3
+            // block, and the flow's four texels lie in the frame
+            const bool interior = ((X - 2) >> 1) >= g.cx0 && ((X + 2) >> 1) <= g.cx1 && ((Y - 2) >> 1) >= g.cy0 && ((Y + 2) >> 1) <= g.cy1 &&
+                                  g.cx1 - g.cx0 >= 2 && g.cy1 - g.cy0 >= 2 && p.ib >= 0 && p.ib + 1 < g.W && p.jb >= 0 && p.jb + 1 < g.H &&
+                                  wmax < 1e30f;
+            for (int f = 0;; f++) {
+                switch (Y & 3) {  // the same for the whole CTA
+                case 0: f = frames_x2<0, SANE>(A, f, x, y, w, interior, a, ws); break;
+                case 1: f = frames_x2<1, SANE>(A, f, x, y, w, interior, a, ws); break;
+                case 2: f = frames_x2<2, SANE>(A, f, x, y, w, interior, a, ws); break;
+                default: f = frames_x2<3, SANE>(A, f, x, y, w, interior, a, ws); break;
+                }
+                if (f >= A.nframes) break;
+                const Sums s = frame_per_tap(A, f, x, y);
 #pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (k == c) { Wc[k] += wc; Ac[k] = fmaf(wc, raw, Ac[k]); }
+                for (int c = 0; c < 3; c++) {
+                    a[c] += (s.a[c] - A.black.v[c] * s.w[c]) * A.rwhite.v[c];
+                    ws[c] += s.w[c];
                 }
             }
         }
 #pragma unroll
-        for (int cc = 0; cc < 3; cc++) {
-            a[cc] += (Ac[cc] - A.black.v[cc] * Wc[cc]) * A.rwhite.v[cc];
-            ws[cc] += Wc[cc];
-        }
+        for (int c = 0; c < 3; c++) { so[part][0][3 * lx + c] = a[c]; so[part][1][3 * lx + c] = ws[c]; }
     }
-    ap[0] = a[0]; ap[1] = a[1]; ap[2] = a[2];
-    wp[0] = ws[0]; wp[1] = ws[1]; wp[2] = ws[2];
-}
-
-template <bool SANE>
-__global__ void __launch_bounds__(256, SANE ? 3 : 2) k_accumulate_x2(const X2Args A)
-{
-    const int ph = blockIdx.x & 3, rph = blockIdx.y & 3;
-    const int x = (blockIdx.x >> 2) * 128 + 4 * threadIdx.x + ph;
-    const int y = A.g.yb0 + (blockIdx.y >> 2) * 32 + 4 * threadIdx.y + rph;
-    if (x >= A.g.Wo || y >= A.g.yb1) return;
-    // X mod 4 and Y mod 4 are the same for the whole CTA
-    switch (((ph + A.g.ox) & 3) | (((rph + A.g.oy) & 3) << 2)) {
-#define ISA_X2_CASE(k) \
-    case k: pixel_x2<((k) & 3), ((k) >> 2), SANE>(A, x, y); break;
-        ISA_X2_CASE(0) ISA_X2_CASE(1) ISA_X2_CASE(2) ISA_X2_CASE(3) ISA_X2_CASE(4) ISA_X2_CASE(5) ISA_X2_CASE(6) ISA_X2_CASE(7)
-        ISA_X2_CASE(8) ISA_X2_CASE(9) ISA_X2_CASE(10) ISA_X2_CASE(11) ISA_X2_CASE(12) ISA_X2_CASE(13) ISA_X2_CASE(14) ISA_X2_CASE(15)
-#undef ISA_X2_CASE
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int i = tid + k * X2_W;
+        if (i < nx) { arow[i] = so[part][0][i]; wrow[i] = so[part][1][i]; }
     }
 }
 
@@ -316,33 +415,36 @@ bool bayer_of(unsigned cfa, Bayer& b)
 
 }  // namespace
 
-bool isa_accumulate_x2_supported(unsigned cfa)
+// Frames whose byte offsets fit 32 bits (the kernel's address arithmetic), and a Bayer layout.
+bool isa_accumulate_x2_supported(const isa_accum_geom& g, unsigned cfa, int nframes, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch)
 {
     Bayer b;
-    return bayer_of(cfa, b);
+    const unsigned long long lim = 1ull << 32, H = (unsigned long long)g.H;
+    return bayer_of(cfa, b) && nframes <= ISA_ACC_MAX_FRAMES && g.W >= 4 && g.H >= 4 && H * raw_pitch < lim && H * flow_pitch < lim &&
+           H / 2 * mask_pitch < lim;
 }
 
-cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, const isa_frame_in* single,
-                                     size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch,
-                                     const float* white, const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into,
-                                     cudaStream_t st)
+cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, size_t raw_pitch,
+                                     size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch, const float* white,
+                                     const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into, cudaStream_t st)
 {
     X2Args A;
-    if (!bayer_of(cfa, A.bayer)) return cudaErrorInvalidValue;
+    if (!bayer_of(cfa, A.bayer) || nframes < 0 || nframes > ISA_ACC_MAX_FRAMES) return cudaErrorInvalidValue;
     A.g = g;
     A.cfa = cfa;
-    A.frames = frames;
     A.nframes = nframes;
-    A.single = single ? *single : isa_frame_in{nullptr, nullptr, nullptr};
+    for (int f = 0; f < nframes; f++) A.frames[f] = frames[f];
     A.raw_pitch = raw_pitch; A.flow_pitch = flow_pitch; A.mask_pitch = mask_pitch;
     A.kparam = (const float4*)kparam; A.kp_pitch = kparam_pitch;
     for (int c = 0; c < 3; c++) { A.rwhite.v[c] = (float)(1.0 / (double)white[c]); A.black.v[c] = black[c]; }
     A.acc = acc; A.wsum = wsum; A.out_pitch = out_pitch; A.accumulate_into = accumulate_into;
     if (g.yb0 % 32 || g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
-    dim3 b(32, 8), grd(((g.Wo + 127) / 128) * 4, ((g.yb1 - g.yb0 + 31) / 32) * 4);
+    const long long blocks = (long long)((g.Wo + X2_W - 1) / X2_W) * ((g.yb1 - g.yb0 + 31) / 32 * 8);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const unsigned grd = (unsigned)blocks;
     if (g.masks_finite)
-        k_accumulate_x2<true><<<grd, b, 0, st>>>(A);
+        k_accumulate_x2<true><<<grd, X2_NT, 0, st>>>(A);
     else
-        k_accumulate_x2<false><<<grd, b, 0, st>>>(A);
+        k_accumulate_x2<false><<<grd, X2_NT, 0, st>>>(A);
     return cudaGetLastError();
 }
