@@ -579,8 +579,8 @@ cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const i
                                   int kparam_channels, const float* white, const float* black, float* acc, float* wsum, size_t out_pitch,
                                   int accumulate_into, cudaStream_t st)
 {
-    if (!g.bilinear && g.s_int == 2 && kparam_channels == 4 && isa_accumulate_x2_supported(g, cfa, nframes, raw_pitch, flow_pitch, mask_pitch))
-        return isa_launch_accumulate_x2(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc, wsum,
+    if (!g.bilinear && kparam_channels == 4 && isa_accumulate_bayer_supported(g, cfa, nframes, raw_pitch, flow_pitch, mask_pitch))
+        return isa_launch_accumulate_bayer(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc, wsum,
                                         out_pitch, accumulate_into, st);
     if (nframes > 1 && !frames_dev) return cudaErrorInvalidValue;
     F3 wh, bl;

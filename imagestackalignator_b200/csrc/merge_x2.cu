@@ -1,6 +1,6 @@
-// Kernel-weighted Bayer accumulation at merge scale 2 (the reference's
+// Kernel-weighted Bayer accumulation at merge scales 2 (the reference's
 // accumulateImagesSuperRes, DeBayerKernels.cu:379-468, and its whole-frame
-// generalisation), restructured so that no lane of a warp diverges from the
+// generalisation) and 1 (accumulateImages, :290-376; below), restructured so that no lane of a warp diverges from the
 // others on the interior path.
 //
 // Geometry at s = 2. Output pixel (X, Y) (origin included) with shift
@@ -142,9 +142,9 @@ struct X2Args {
     isa_frame_in frames[ISA_ACC_MAX_FRAMES];
 };
 
-// What a frame without flow or mask reads, at offset 0.
+// What a frame without flow (two texels) or mask (up to three cells) reads, at offset 0.
 __device__ const float4 g_zero_flow = {0.f, 0.f, 0.f, 0.f};
-__device__ const float4 g_unit_mask[2] = {{1.f, 1.f, 1.f, 1.f}, {1.f, 1.f, 1.f, 1.f}};
+__device__ const float4 g_unit_mask[3] = {{1.f, 1.f, 1.f, 1.f}, {1.f, 1.f, 1.f, 1.f}, {1.f, 1.f, 1.f, 1.f}};
 
 struct Sums { float a[3], w[3]; };
 
@@ -193,13 +193,15 @@ __device__ __forceinline__ float tap_weights(float k0, float k1, float k2, float
     return wmax;
 }
 
-// One frame's sums of a pixel tap by tap, with the crop clamps and mirrored flow of the reference.
+// One frame's sums of a pixel tap by tap at scale S (1 or 2), with the crop clamps and mirrored flow of the reference.
+template <int S>
 __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
 {
+    constexpr int SH = S - 1;
     const isa_accum_geom& g = A.g;
     const isa_frame_in fr = A.frames[f];
-    const Position p = position(g, x, y);
     const int X = x + g.ox, Y = y + g.oy;
+    const Position p = S == 1 ? Position{X, Y, 0.f, 0.f} : position(g, x, y);
     float k0, k1, k2, w[5][5];
     kernel_params(A, p, k0, k1, k2);
     tap_weights(k0, k1, k2, w);
@@ -210,19 +212,19 @@ __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
         const float2* r0 = isa::row_ptr(fr.flow, A.flow_pitch, isa::mirror(p.jb, g.H));
         const float2* r1 = isa::row_ptr(fr.flow, A.flow_pitch, isa::mirror(p.jb + 1, g.H));
         const float2 p00 = __ldg(r0 + i0), p10 = __ldg(r0 + i1), p01 = __ldg(r1 + i0), p11 = __ldg(r1 + i1);
-        sx = (int)roundf(isa::lerp2(p00.x, p10.x, p01.x, p11.x, p.ax, p.by) * 2.0f);
-        sy = (int)roundf(isa::lerp2(p00.y, p10.y, p01.y, p11.y, p.ax, p.by) * 2.0f);
+        sx = (int)roundf(isa::lerp2(p00.x, p10.x, p01.x, p11.x, p.ax, p.by) * (float)S);
+        sy = (int)roundf(isa::lerp2(p00.y, p10.y, p01.y, p11.y, p.ax, p.by) * (float)S);
     }
     int qx[5], ux[5];
 #pragma unroll
     for (int d = 0; d < 5; d++) {
-        qx[d] = isa::clampi((X + sx + d - 2) >> 1, g.cx0, g.cx1);
-        ux[d] = (isa::clampi((X + d - 2) >> 1, g.cx0, g.cx1) >> 1) * 4;
+        qx[d] = isa::clampi((X + sx + d - 2) >> SH, g.cx0, g.cx1);
+        ux[d] = (isa::clampi((X + d - 2) >> SH, g.cx0, g.cx1) >> 1) * 4;
     }
 #pragma unroll
     for (int py = -2; py <= 2; py++) {
-        const int qy = isa::clampi((Y + sy + py) >> 1, g.cy0, g.cy1);
-        const int uy = isa::clampi((Y + py) >> 1, g.cy0, g.cy1) >> 1;
+        const int qy = isa::clampi((Y + sy + py) >> SH, g.cy0, g.cy1);
+        const int uy = isa::clampi((Y + py) >> SH, g.cy0, g.cy1) >> 1;
         const uint16_t* rr = isa::row_ptr(fr.raw, A.raw_pitch, qy);
         const float* mr = fr.mask ? (const float*)isa::row_ptr(fr.mask, A.mask_pitch, uy) : nullptr;
 #pragma unroll
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
                 default: f = frames_x2<3, SANE>(A, f, x, y, w, interior, a, ws); break;
                 }
                 if (f >= A.nframes) break;
-                const Sums s = frame_per_tap(A, f, x, y);
+                const Sums s = frame_per_tap<2>(A, f, x, y);
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     a[c] += (s.a[c] - A.black.v[c] * s.w[c]) * A.rwhite.v[c];
@@ -392,6 +394,135 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
         const int i = tid + k * X2_W;
         if (i < nx) { arow[i] = so[part][0][i]; wrow[i] = so[part][1][i]; }
     }
+}
+
+// ---- scale 1 (accumulateImages) ------------------------------------------------
+// Output pixel (X, Y) reads the 5 x 5 samples around (X + sx, Y + sy), each
+// with the certainty of the unshifted tap's mask cell: 3 x 3 cells, the taps
+// of a line on cells 0 0 1 1 2 where X is even and 0 1 1 2 2 where it is odd.
+// Relative to the block's first sample a tap's CFA class is its own parity, a
+// compile-time constant; the certainty of a class is one of two values per
+// mask cell and row parity. Row patterns (YM = Y mod 2) are a template
+// parameter, uniform in a CTA; the column pattern is a select per lane.
+// Bound: instruction issue, 75 multiply-adds and about as many selects and
+// loads per pixel and frame. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
+// with its clamps, divisions and indexed channels; one 3010x2006 frame by
+// itself 0.22 ms, from 0.72 ms. CTAs of 512 threads: 2.9 ms and 0.24 ms; at 80
+// registers (24 warps per SM) 3.0 ms.
+constexpr int X1_NT = 2 * X2_W, X1_CTAS = 4;
+
+template <int YM, bool SANE>
+__device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, const float (&w)[5][5], bool interior, float (&a)[3], float (&ws)[3])
+{
+    const isa_accum_geom& g = A.g;
+    const unsigned foff = (unsigned)isa::clampi(Y, 0, g.H - 1) * (unsigned)A.flow_pitch + (unsigned)isa::clampi(X, 0, g.W - 1) * 8u;
+    const unsigned moff = (unsigned)isa::clampi((Y - 2) >> 1, 0, g.H / 2 - 1) * (unsigned)A.mask_pitch + (unsigned)isa::clampi((X - 2) >> 1, 0, g.W / 2 - 1) * 16u;
+    // the shifted 5 x 5 block lies inside the crop
+    const unsigned kspan = (unsigned)(g.cx1 - 4 - g.cx0), jspan = (unsigned)(g.cy1 - 4 - g.cy0);
+    const bool odd = X & 1;
+    int f = f0;
+#pragma unroll 1
+    for (; f < A.nframes; f++) {
+        int sx = 0, sy = 0;
+        if (A.frames[f].flow) {
+            const float2 fl = __ldg((const float2*)((const char*)A.frames[f].flow + foff));
+            sx = (int)roundf(fl.x);
+            sy = (int)roundf(fl.y);
+        }
+        const int k0 = X + sx - 2, j0 = Y + sy - 2;
+        if (!(interior && (unsigned)(k0 - g.cx0) <= kspan && (unsigned)(j0 - g.cy0) <= jspan)) break;
+        const unsigned ro = (unsigned)j0 * (unsigned)A.raw_pitch + 2u * (unsigned)k0;
+        const char* mk = (const char*)A.frames[f].mask;
+        const unsigned mo = mk ? moff : 0u;
+        const size_t mp = mk ? A.mask_pitch : 0;
+        const char* mb = mk ? mk : (const char*)g_unit_mask;
+        const bool fx = k0 & 1, fy = j0 & 1;
+        const bool hG = (int)(fx ^ fy) == A.bayer.g0, frr = (int)fy == A.bayer.ry;
+        float Ac[4] = {0.f, 0.f, 0.f, 0.f}, Wc[4] = {0.f, 0.f, 0.f, 0.f};
+        float4 M[3];
+#pragma unroll
+        for (int r = 0; r < 5; r++) {
+            constexpr int MR[2][5] = {{0, 0, 1, 1, 2}, {0, 1, 1, 2, 2}};
+            if (r == 0 || MR[YM][r] != MR[YM][r > 0 ? r - 1 : 0]) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    M[c] = __ldg((const float4*)(mb + MR[YM][r] * mp + mo) + c);
+                    if (!SANE) M[c] = sanitize(M[c]);
+                }
+            }
+            const int rp = r & 1;
+            const bool red = rp ? !frr : frr, gE = rp ? !hG : hG;  // the row's other colour; green on its even taps
+            float E[3], O[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float rb = red ? M[c].x : M[c].z;
+                E[c] = gE ? M[c].y : rb;
+                O[c] = gE ? rb : M[c].y;
+            }
+            const float k[5] = {E[0], odd ? O[1] : O[0], E[1], odd ? O[2] : O[1], E[2]};
+            const uint16_t* rr = (const uint16_t*)((const char*)A.frames[f].raw + r * A.raw_pitch + ro);
+#pragma unroll
+            for (int d = 0; d < 5; d++) {
+                const float wc = __fmul_rn(w[r][d], k[d]);
+                const int cl = rp * 2 + (d & 1);
+                Ac[cl] = __fmaf_rn(wc, (float)__ldg(rr + d), Ac[cl]);
+                Wc[cl] = __fadd_rn(Wc[cl], wc);
+            }
+        }
+        // relative classes -> R, G, B
+        const float NA0 = hG ? Ac[1] : Ac[0], NA1 = hG ? Ac[2] : Ac[3], NW0 = hG ? Wc[1] : Wc[0], NW1 = hG ? Wc[2] : Wc[3];
+        const float ga = (hG ? Ac[0] : Ac[1]) + (hG ? Ac[3] : Ac[2]), gw = (hG ? Wc[0] : Wc[1]) + (hG ? Wc[3] : Wc[2]);
+        const float ra = frr ? NA0 : NA1, ba = frr ? NA1 : NA0, rw = frr ? NW0 : NW1, bw = frr ? NW1 : NW0;
+        a[0] = __fmaf_rn(__fmaf_rn(-A.black.v[0], rw, ra), A.rwhite.v[0], a[0]);
+        a[1] = __fmaf_rn(__fmaf_rn(-A.black.v[1], gw, ga), A.rwhite.v[1], a[1]);
+        a[2] = __fmaf_rn(__fmaf_rn(-A.black.v[2], bw, ba), A.rwhite.v[2], a[2]);
+        ws[0] += rw;
+        ws[1] += gw;
+        ws[2] += bw;
+    }
+    return f;
+}
+
+template <bool SANE>
+__global__ void __launch_bounds__(X1_NT, X1_CTAS) k_accumulate_x1(const __grid_constant__ X2Args A)
+{
+    const isa_accum_geom& g = A.g;
+    // CTA rows in bands of four output rows: the two even rows, then the two odd ones
+    const int nbx = (g.Wo + X2_W - 1) / X2_W;
+    const int row = blockIdx.x / nbx;
+    const int x = (blockIdx.x - row * nbx) * X2_W + threadIdx.x % X2_W;
+    const int y = g.yb0 + 4 * (row >> 1) + 2 * (threadIdx.x / X2_W) + (row & 1);
+    if (x >= g.Wo || y >= g.yb1) return;
+    float* ap = isa::row_ptr(A.acc, A.out_pitch, y) + 3 * x;
+    float* wp = isa::row_ptr(A.wsum, A.out_pitch, y) + 3 * x;
+    if (x < 1 || y < 1 || x >= g.Wo - 1 || y >= g.Ho - 1) {
+        if (!A.accumulate_into) { ap[0] = ap[1] = ap[2] = 0.f; wp[0] = wp[1] = wp[2] = 0.f; }
+        return;
+    }
+    float a[3] = {0.f, 0.f, 0.f}, ws[3] = {0.f, 0.f, 0.f};
+    if (A.accumulate_into) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) { a[c] = ap[c]; ws[c] = wp[c]; }
+    }
+    const int X = x + g.ox, Y = y + g.oy;
+    const float4 kp = __ldg(isa::row_ptr(A.kparam, A.kp_pitch, isa::clampi(Y, 0, g.H - 1)) + isa::clampi(X, 0, g.W - 1));
+    float w[5][5];
+    const float wmax = tap_weights(kp.x, kp.y, kp.z, w);
+    // the unshifted taps lie inside the crop (and with them the flow's texel in the frame), the crop holds a 5 x 5 block
+    const bool interior = X - 2 >= g.cx0 && X + 2 <= g.cx1 && Y - 2 >= g.cy0 && Y + 2 <= g.cy1 && wmax < 1e30f;
+    for (int f = 0;; f++) {
+        if ((Y & 1) == 0) f = frames_x1<0, SANE>(A, f, X, Y, w, interior, a, ws);  // the same for the whole CTA
+        else f = frames_x1<1, SANE>(A, f, X, Y, w, interior, a, ws);
+        if (f >= A.nframes) break;
+        const Sums s = frame_per_tap<1>(A, f, x, y);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            a[c] += (s.a[c] - A.black.v[c] * s.w[c]) * A.rwhite.v[c];
+            ws[c] += s.w[c];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) { ap[c] = a[c]; wp[c] = ws[c]; }
 }
 
 // The CFA is a Bayer pattern: codes 0/1/2 only, the two greens on one
@@ -415,18 +546,18 @@ bool bayer_of(unsigned cfa, Bayer& b)
 
 }  // namespace
 
-// Frames whose byte offsets fit 32 bits (the kernel's address arithmetic), and a Bayer layout.
-bool isa_accumulate_x2_supported(const isa_accum_geom& g, unsigned cfa, int nframes, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch)
+// Merge scales 1 and 2 of a Bayer layout, frames whose byte offsets fit 32 bits (the kernels' address arithmetic).
+bool isa_accumulate_bayer_supported(const isa_accum_geom& g, unsigned cfa, int nframes, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch)
 {
     Bayer b;
     const unsigned long long lim = 1ull << 32, H = (unsigned long long)g.H;
-    return bayer_of(cfa, b) && nframes <= ISA_ACC_MAX_FRAMES && g.W >= 4 && g.H >= 4 && H * raw_pitch < lim && H * flow_pitch < lim &&
-           H / 2 * mask_pitch < lim;
+    return (g.s_int == 1 || g.s_int == 2) && bayer_of(cfa, b) && nframes <= ISA_ACC_MAX_FRAMES && g.W >= 4 && g.H >= 4 && H * raw_pitch < lim &&
+           H * flow_pitch < lim && H / 2 * mask_pitch < lim;
 }
 
-cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, size_t raw_pitch,
-                                     size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch, const float* white,
-                                     const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into, cudaStream_t st)
+cudaError_t isa_launch_accumulate_bayer(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, int nframes, size_t raw_pitch,
+                                        size_t flow_pitch, size_t mask_pitch, const float* kparam, size_t kparam_pitch, const float* white,
+                                        const float* black, float* acc, float* wsum, size_t out_pitch, int accumulate_into, cudaStream_t st)
 {
     X2Args A;
     if (!bayer_of(cfa, A.bayer) || nframes < 0 || nframes > ISA_ACC_MAX_FRAMES) return cudaErrorInvalidValue;
@@ -439,12 +570,11 @@ cudaError_t isa_launch_accumulate_x2(const isa_accum_geom& g, unsigned cfa, cons
     for (int c = 0; c < 3; c++) { A.rwhite.v[c] = (float)(1.0 / (double)white[c]); A.black.v[c] = black[c]; }
     A.acc = acc; A.wsum = wsum; A.out_pitch = out_pitch; A.accumulate_into = accumulate_into;
     if (g.yb0 % 32 || g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
-    const long long blocks = (long long)((g.Wo + X2_W - 1) / X2_W) * ((g.yb1 - g.yb0 + 31) / 32 * 8);
+    const int rows = g.yb1 - g.yb0;  // CTA rows: four rows each in bands of 32, or two each in bands of 4
+    const long long blocks = (long long)((g.Wo + X2_W - 1) / X2_W) * (g.s_int == 2 ? (rows + 31) / 32 * 8 : (rows + 3) / 4 * 2);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const unsigned grd = (unsigned)blocks;
-    if (g.masks_finite)
-        k_accumulate_x2<true><<<grd, X2_NT, 0, st>>>(A);
-    else
-        k_accumulate_x2<false><<<grd, X2_NT, 0, st>>>(A);
+    const auto kernel = g.s_int == 2 ? (g.masks_finite ? k_accumulate_x2<true> : k_accumulate_x2<false>)
+                                     : (g.masks_finite ? k_accumulate_x1<true> : k_accumulate_x1<false>);
+    kernel<<<(unsigned)blocks, g.s_int == 2 ? X2_NT : X1_NT, 0, st>>>(A);
     return cudaGetLastError();
 }

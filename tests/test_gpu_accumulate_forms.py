@@ -1,6 +1,6 @@
 """The accumulation's specialised kernels against its general one over the forms
 both accept: the same call with 4-channel kernel parameters (specialised at
-scale 2) and with 3-channel ones (always the general, tap-by-tap kernel).
+scales 1 and 2) and with 3-channel ones (always the general, tap-by-tap kernel).
 
 Tolerance: a frame adds at most 25 products per channel in a chain of FP32
 multiply-adds, folds and a final scaling, under 32 roundings of 2^-24 relative
@@ -44,6 +44,16 @@ CASES = [
     (16, 16, 2.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 1.0, "zero"),
     (4, 4, 2.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 0.5, "rand"),
     (2, 2, 2.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 0.5, "rand"),
+    (130, 66, 1.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 3.0, "rand"),
+    (258, 34, 1.0, 0, 0, None, 257, 33, (2, 1, 1, 0), 40.0, "rand"),
+    (64, 34, 1.0, 7, 5, (9, 6, 50, 30), 50, 27, (1, 0, 2, 1), 2.0, "rand"),    # odd origin and crop
+    (64, 34, 1.0, -3, -2, None, 70, 40, (1, 2, 0, 1), 1.0, "nonfinite"),       # output beyond the frame
+    (64, 64, 1.0, 0, 0, None, 0, 0, (0, 1, 1, 2), None, None),
+    (64, 64, 1.0, 0, 0, None, 0, 0, (1, 2, 0, 1), 2.0, None),
+    (64, 64, 1.0, 0, 0, (30, 30, 33, 33), 0, 0, (0, 1, 1, 2), 2.0, "rand"),    # a crop smaller than a 5 x 5 block
+    (16, 16, 1.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 1.0, "zero"),
+    (4, 4, 1.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 0.5, "rand"),
+    (2, 2, 1.0, 0, 0, None, 0, 0, (0, 1, 1, 2), 0.5, "rand"),
 ]
 
 
