@@ -113,12 +113,119 @@ __device__ __forceinline__ float2 flow_sample(const float2* fl, size_t pitch, in
     return make_float2(isa::lerp2(p00.x, p10.x, p01.x, p11.x, a, b), isa::lerp2(p00.y, p10.y, p01.y, p11.y, a, b));
 }
 
-// BIL (sample mode BILINEAR): each frame contributes at the four integer
+// floor((float)v / g.s), the quotient rounded to FP32, without the division: the nearest integer c to v (1 / s) is off by
+// less than one, and the sign of v - c s (exact in one multiply-add) tells on which side of c the quotient lies. Only a
+// quotient below c by less than half an FP32 step would round up to it: there, the division decides.
+__device__ __forceinline__ int floor_div_f(int v, float s, float rs)
+{
+    const float fv = (float)v, c = rintf(fv * rs), e = fmaf(-c, s, fv);
+    if (e < 0.f && e > fabsf(c) * s * -0x1p-22f) return (int)floorf(fv / s);
+    return (int)(e < 0.f ? c - 1.f : c);
+}
+
+// Any scale and CFA, tap by tap: the row and column of a tap give its sample, mask cell and CFA class (row and column
+// parity); a frame's sums are kept per class, the two classes of a row apart by predicates, and go to the channels and
+// through the black and white levels once per frame. The division by s is floor_div_f, exact where the taps' positions
+// are below 2^22 (|v| < 2^22: the frames of isa_ctx_create's limits at scale 8 stay below 2^18).
+// Bound: instruction issue, about 1200 instructions per pixel and frame, mostly address arithmetic and predicated sums.
+// 6 x 2000x1500 at 1.5x: 1.8 ms, from 5.4 ms with per-tap divisions, indexed channels and normalisation.
+template <int KC>
+__global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
+                                                      isa_frame_in single, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch,
+                                                      const float* __restrict__ kparam, size_t kp_pitch, F3 rwhite, F3 black, float* __restrict__ acc,
+                                                      float* __restrict__ wsum, size_t out_pitch, int accumulate_into)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = g.yb0 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= g.Wo || y >= g.yb1) return;
+    float* ap = isa::row_ptr(acc, out_pitch, y) + 3 * x;
+    float* wp = isa::row_ptr(wsum, out_pitch, y) + 3 * x;
+    if (x < 1 || y < 1 || x >= g.Wo - 1 || y >= g.Ho - 1) {
+        if (!accumulate_into) { ap[0] = ap[1] = ap[2] = 0.f; wp[0] = wp[1] = wp[2] = 0.f; }
+        return;
+    }
+    float a[3] = {0.f, 0.f, 0.f}, w[3] = {0.f, 0.f, 0.f};
+    if (accumulate_into) {
+        a[0] = ap[0]; a[1] = ap[1]; a[2] = ap[2];
+        w[0] = wp[0]; w[1] = wp[1]; w[2] = wp[2];
+    }
+    const float xb = ((float)x + 0.5f + (float)g.ox) / g.s - 0.5f;
+    const float yb = ((float)y + 0.5f + (float)g.oy) / g.s - 0.5f;
+    const float rs = 1.f / g.s;
+    float k[3];
+    kparam_sample<KC>(kparam, kp_pitch, g.W, g.H, xb, yb, k);
+    float wt[25];
+#pragma unroll
+    for (int py = -2; py <= 2; py++)
+#pragma unroll
+        for (int px = -2; px <= 2; px++) {
+            float q = px * px * k[0] + 2 * px * py * k[2] + py * py * k[1];
+            float v = expf(-0.5f * q);
+            if (!isfinite(v)) v = px * py == 0 ? 1.f : 0.f;
+            wt[(py + 2) * 5 + px + 2] = v;
+        }
+    // unshifted taps (mask rows and columns, in floats) do not depend on the frame
+    int ux[5], uy[5];
+#pragma unroll
+    for (int d = 0; d < 5; d++) {
+        ux[d] = (isa::clampi(floor_div_f(x + d - 2 + g.ox, g.s, rs), g.cx0, g.cx1) >> 1) * 4;
+        uy[d] = isa::clampi(floor_div_f(y + d - 2 + g.oy, g.s, rs), g.cy0, g.cy1) >> 1;
+    }
+#pragma unroll 1
+    for (int f = 0; f < nframes; f++) {
+        const isa_frame_in fr = frames ? frames[f] : single;
+        int sx0 = 0, sy0 = 0;
+        if (fr.flow) {
+            const float2 fl = flow_sample(fr.flow, flow_pitch, g.W, g.H, xb, yb);
+            sx0 = (int)roundf(fl.x * g.s);
+            sy0 = (int)roundf(fl.y * g.s);
+        }
+        int qx[5];
+#pragma unroll
+        for (int d = 0; d < 5; d++) qx[d] = isa::clampi(floor_div_f(x + d - 2 + sx0 + g.ox, g.s, rs), g.cx0, g.cx1);
+        float A[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, W[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [row parity][column parity]
+#pragma unroll
+        for (int py = 0; py < 5; py++) {
+            const int qy = isa::clampi(floor_div_f(y + py - 2 + sy0 + g.oy, g.s, rs), g.cy0, g.cy1);
+            const uint16_t* rr = isa::row_ptr(fr.raw, raw_pitch, qy);
+            const float* mr = fr.mask ? (const float*)isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
+            const unsigned codes = cfa >> ((qy & 1) * 4);  // of the row's even and odd columns
+            const int ce = codes & 3, co = (codes >> 2) & 3;
+            float ae = 0.f, ao = 0.f, we = 0.f, wo = 0.f;
+#pragma unroll
+            for (int px = 0; px < 5; px++) {
+                const bool odd = qx[px] & 1;
+                float cert = 1.f;
+                if (mr) {
+                    cert = __ldg(mr + (ux[px] + (odd ? co : ce)));
+                    if (!isfinite(cert)) cert = 0.f;
+                }
+                const float wc = __fmul_rn(wt[py * 5 + px], cert), raw = (float)__ldg(rr + qx[px]);
+                if (odd) { wo = __fadd_rn(wo, wc); ao = __fmaf_rn(wc, raw, ao); }
+                else { we = __fadd_rn(we, wc); ae = __fmaf_rn(wc, raw, ae); }
+            }
+            if (qy & 1) { W[1][0] += we; W[1][1] += wo; A[1][0] += ae; A[1][1] += ao; }
+            else { W[0][0] += we; W[0][1] += wo; A[0][0] += ae; A[0][1] += ao; }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            float sa = 0.f, sw = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (((cfa >> (2 * q)) & 3) == (unsigned)c) { sa += A[q >> 1][q & 1]; sw += W[q >> 1][q & 1]; }
+            a[c] = __fmaf_rn(__fmaf_rn(-black.v[c], sw, sa), rwhite.v[c], a[c]);
+            w[c] += sw;
+        }
+    }
+    ap[0] = a[0]; ap[1] = a[1]; ap[2] = a[2];
+    wp[0] = w[0]; wp[1] = w[1]; wp[2] = w[2];
+}
+
+// Sample mode BILINEAR: each frame contributes at the four integer
 // shifts around s * flow with the bilinear weights of its fractional part
 // (the certainty of a tap is scaled by the corner's weight); corners of
 // weight zero are skipped, so at integer flow the sums are ROUND's.
-template <int KC, bool BIL>
-__global__ void __launch_bounds__(256) k_accumulate(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
+template <int KC>
+__global__ void __launch_bounds__(256) k_accumulate_bil(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
                                                    isa_frame_in single, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* __restrict__ kparam,
                                                    size_t kp_pitch, F3 white, F3 black, float* __restrict__ acc, float* __restrict__ wsum,
                                                    size_t out_pitch, int accumulate_into)
@@ -163,74 +270,43 @@ __global__ void __launch_bounds__(256) k_accumulate(isa_accum_geom g, unsigned c
         float bx = 0.f, by = 0.f;
         if (fr.flow) {
             float2 fl = flow_sample(fr.flow, flow_pitch, g.W, g.H, xb, yb);
-            if constexpr (BIL) {
-                const float hx = fl.x * g.s, hy = fl.y * g.s;
-                const float fx = floorf(hx), fy = floorf(hy);
-                sx0 = (int)fx; sy0 = (int)fy;
-                bx = hx - fx; by = hy - fy;
-            } else {
-                sx0 = (int)roundf(fl.x * g.s);
-                sy0 = (int)roundf(fl.y * g.s);
-            }
+            const float hx = fl.x * g.s, hy = fl.y * g.s;
+            const float fx = floorf(hx), fy = floorf(hy);
+            sx0 = (int)fx; sy0 = (int)fy;
+            bx = hx - fx; by = hy - fy;
         }
-        if constexpr (BIL) {
-            // the four corners' taps fall on 6 x 6 output-grid positions: their source rows, columns and CFA
-            // colours once; each tap's mask cell (the unshifted tap's) is shared by the corners
-            const float wk[4] = {(1.f - bx) * (1.f - by), bx * (1.f - by), (1.f - bx) * by, bx * by};
-            int qxs[6];
-            const uint16_t* rrs[6];
-            int qys[6];
+        // the four corners' taps fall on 6 x 6 output-grid positions: their source rows, columns and CFA
+        // colours once; each tap's mask cell (the unshifted tap's) is shared by the corners
+        const float wk[4] = {(1.f - bx) * (1.f - by), bx * (1.f - by), (1.f - bx) * by, bx * by};
+        int qxs[6];
+        const uint16_t* rrs[6];
+        int qys[6];
 #pragma unroll
-            for (int d = 0; d < 6; d++) {
-                qxs[d] = isa::clampi(floor_div_s(x + d - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
-                qys[d] = isa::clampi(floor_div_s(y + d - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
-                rrs[d] = isa::row_ptr(fr.raw, raw_pitch, qys[d]);
-            }
+        for (int d = 0; d < 6; d++) {
+            qxs[d] = isa::clampi(floor_div_s(x + d - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
+            qys[d] = isa::clampi(floor_div_s(y + d - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
+            rrs[d] = isa::row_ptr(fr.raw, raw_pitch, qys[d]);
+        }
 #pragma unroll
-            for (int py = 0; py < 5; py++) {
-                const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
+        for (int py = 0; py < 5; py++) {
+            const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
 #pragma unroll
-                for (int px = 0; px < 5; px++) {
-                    float4 m = make_float4(1.f, 1.f, 1.f, 1.f);
-                    if (mr) m = __ldg(mr + ux[px]);
-                    const float ww = wt[py * 5 + px];
+            for (int px = 0; px < 5; px++) {
+                float4 m = make_float4(1.f, 1.f, 1.f, 1.f);
+                if (mr) m = __ldg(mr + ux[px]);
+                const float ww = wt[py * 5 + px];
 #pragma unroll
-                    for (int corner = 0; corner < 4; corner++) {
-                        if (wk[corner] == 0.f) continue;
-                        const int dx = corner & 1, dy = corner >> 1;
-                        const int qx = qxs[px + dx], qy = qys[py + dy];
-                        const int c = isa::cfa_at(cfa, qx, qy);
-                        if (c > 2) continue;
-                        float raw = (float)__ldg(rrs[py + dy] + qx);
-                        raw = (raw - black.v[c]) / white.v[c];
-                        float cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
-                        if (!isfinite(cert)) cert = 0.f;
-                        cert *= wk[corner];
-                        a[c] += raw * ww * cert;
-                        w[c] += ww * cert;
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int py = 0; py < 5; py++) {
-                const int qy = isa::clampi(floor_div_s(y + py - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
-                const uint16_t* rr = isa::row_ptr(fr.raw, raw_pitch, qy);
-                const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
-#pragma unroll
-                for (int px = 0; px < 5; px++) {
-                    const int qx = isa::clampi(floor_div_s(x + px - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
+                for (int corner = 0; corner < 4; corner++) {
+                    if (wk[corner] == 0.f) continue;
+                    const int dx = corner & 1, dy = corner >> 1;
+                    const int qx = qxs[px + dx], qy = qys[py + dy];
                     const int c = isa::cfa_at(cfa, qx, qy);
                     if (c > 2) continue;
-                    float raw = (float)__ldg(rr + qx);
+                    float raw = (float)__ldg(rrs[py + dy] + qx);
                     raw = (raw - black.v[c]) / white.v[c];
-                    float cert = 1.f;
-                    if (mr) {
-                        float4 m = __ldg(mr + ux[px]);
-                        cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
-                        if (!isfinite(cert)) cert = 0.f;
-                    }
-                    const float ww = wt[py * 5 + px];
+                    float cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
+                    if (!isfinite(cert)) cert = 0.f;
+                    cert *= wk[corner];
                     a[c] += raw * ww * cert;
                     w[c] += ww * cert;
                 }
@@ -293,8 +369,150 @@ __device__ __forceinline__ void flow_scatter(float2* gflow, size_t pitch, int W,
     }
 }
 
-template <int KC, bool BIL>
-__global__ void __launch_bounds__(256, 2) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
+// The transpose of the kernel parameters' bilinear lookup (clamp addressing, zero weights skipped as in lerp2): gk
+// scattered to gkp (three floats per texel).
+__device__ __forceinline__ void kparam_scatter(float* gkp, int W, int H, float xb, float yb, const float gk[3])
+{
+    const float fx = floorf(xb), fy = floorf(yb);
+    const int i = (int)fx, j = (int)fy;
+    const float a = xb - fx, b = yb - fy;
+    const int i0 = isa::clampi(i, 0, W - 1), i1 = isa::clampi(i + 1, 0, W - 1), j0 = isa::clampi(j, 0, H - 1), j1 = isa::clampi(j + 1, 0, H - 1);
+    const float w00 = (1.f - a) * (1.f - b), w10 = a * (1.f - b), w01 = (1.f - a) * b, w11 = a * b;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        atomicAdd(gkp + ((size_t)j0 * W + i0) * 3 + c, w00 * gk[c]);
+        if (a != 0.f) atomicAdd(gkp + ((size_t)j0 * W + i1) * 3 + c, w10 * gk[c]);
+        if (b != 0.f) atomicAdd(gkp + ((size_t)j1 * W + i0) * 3 + c, w01 * gk[c]);
+        if (a != 0.f && b != 0.f) atomicAdd(gkp + ((size_t)j1 * W + i1) * 3 + c, w11 * gk[c]);
+    }
+}
+
+// Block sum of the loss, one atomic per block.
+__device__ __forceinline__ void loss_sum(double lsum, double* loss)
+{
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    __shared__ double sl[8];
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    if ((tid & 31) == 0) sl[tid >> 5] = lsum;
+    __syncthreads();
+    if (tid == 0 && loss) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x * blockDim.y) / 32; w++) t += sl[w];
+        atomicAdd(loss, t);
+    }
+}
+
+// Sample mode ROUND. With the black and white levels folded into the pixel's factors (v - out) h =
+// (raw - (black + white out)) (h / white) a tap costs no division; the channel's two factors come per row and column
+// parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
+// Bound: instruction issue and the mask-certainty atomics (one per tap and frame). 6 x 2000x1500 at 1.5x: 3.0 ms, from
+// 8.0 ms with a division and branches on the channel per tap.
+template <int KC>
+__global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
+                                                       size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* __restrict__ kparam,
+                                                       size_t kp_pitch, F3 white, F3 black, const float* __restrict__ out, size_t out_pitch,
+                                                       const float* __restrict__ wsum, size_t ws_pitch, const float* __restrict__ target,
+                                                       size_t tg_pitch, const float* __restrict__ weight, size_t wt_pitch, float* __restrict__ gkp,
+                                                       float4* __restrict__ gmask, size_t gmask_stride, double* __restrict__ loss)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    double lsum = 0.0;
+    if (x < g.Wo && y < g.Ho) {
+        const float* op = isa::row_ptr(out, out_pitch, y) + 3 * x;
+        const float* wp = isa::row_ptr(wsum, ws_pitch, y) + 3 * x;
+        const float* tp = isa::row_ptr(target, tg_pitch, y) + 3 * x;
+        const float om = weight ? isa::row_ptr(weight, wt_pitch, y)[x] : 1.f;
+        float o[3], h[3];  // out in raw units (black + white out), h / white
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const float oc = op[c], d = oc - tp[c];
+            lsum += (double)om * d * d;
+            const float hc = wp[c] != 0.f ? 2.f * om * d / wp[c] : 0.f;
+            any = any || hc != 0.f;
+            o[c] = fmaf(white.v[c], oc, black.v[c]);
+            h[c] = hc / white.v[c];
+        }
+        if (x >= 1 && y >= 1 && x < g.Wo - 1 && y < g.Ho - 1 && any) {
+            const float xb = ((float)x + 0.5f + (float)g.ox) / g.s - 0.5f;
+            const float yb = ((float)y + 0.5f + (float)g.oy) / g.s - 0.5f;
+            const float rs = 1.f / g.s;
+            float k[3];
+            kparam_sample<KC>(kparam, kp_pitch, g.W, g.H, xb, yb, k);
+            float wt[25], G[13];  // G[t]: dL/dw of the taps t and 24 - t
+            bool live[13];
+#pragma unroll
+            for (int t = 0; t < 13; t++) {
+                const int px = t % 5 - 2, py = t / 5 - 2;
+                const float q = px * px * k[0] + 2 * px * py * k[2] + py * py * k[1];
+                float v = expf(-0.5f * q);
+                live[t] = isfinite(v);  // the fallback weight does not depend on k
+                if (!live[t]) v = px * py == 0 ? 1.f : 0.f;
+                wt[t] = wt[24 - t] = v;
+                G[t] = 0.f;
+            }
+            int ux[5], uy[5];
+#pragma unroll
+            for (int d = 0; d < 5; d++) {
+                ux[d] = (isa::clampi(floor_div_f(x + d - 2 + g.ox, g.s, rs), g.cx0, g.cx1) >> 1) * 4;
+                uy[d] = isa::clampi(floor_div_f(y + d - 2 + g.oy, g.s, rs), g.cy0, g.cy1) >> 1;
+            }
+#pragma unroll 1
+            for (int f = 0; f < nframes; f++) {
+                const isa_frame_in fr = frames[f];
+                int sx0 = 0, sy0 = 0;
+                if (fr.flow) {
+                    const float2 fl = flow_sample(fr.flow, flow_pitch, g.W, g.H, xb, yb);
+                    sx0 = (int)roundf(fl.x * g.s);
+                    sy0 = (int)roundf(fl.y * g.s);
+                }
+                float4* gm = gmask + (size_t)f * gmask_stride;
+                int qx[5];
+#pragma unroll
+                for (int d = 0; d < 5; d++) qx[d] = isa::clampi(floor_div_f(x + d - 2 + sx0 + g.ox, g.s, rs), g.cx0, g.cx1);
+#pragma unroll
+                for (int py = 0; py < 5; py++) {
+                    const int qy = isa::clampi(floor_div_f(y + py - 2 + sy0 + g.oy, g.s, rs), g.cy0, g.cy1);
+                    const uint16_t* rr = isa::row_ptr(fr.raw, raw_pitch, qy);
+                    const unsigned codes = cfa >> ((qy & 1) * 4);  // of the row's even and odd columns
+                    const int ce = codes & 3, co = (codes >> 2) & 3;
+                    const float oe = ce == 0 ? o[0] : (ce == 1 ? o[1] : o[2]), he = ce == 0 ? h[0] : (ce == 1 ? h[1] : h[2]);
+                    const float oo = co == 0 ? o[0] : (co == 1 ? o[1] : o[2]), ho = co == 0 ? h[0] : (co == 1 ? h[1] : h[2]);
+                    const size_t mrow = (size_t)uy[py] * mask_pitch;
+#pragma unroll
+                    for (int px = 0; px < 5; px++) {
+                        const int t = py * 5 + px;
+                        const bool odd = qx[px] & 1;
+                        const float r = ((float)__ldg(rr + qx[px]) - (odd ? oo : oe)) * (odd ? ho : he);
+                        float cert = 1.f;
+                        if (fr.mask) {
+                            const size_t at = mrow + 4u * (unsigned)(ux[px] + (odd ? co : ce));
+                            cert = __ldg((const float*)((const char*)fr.mask + at));
+                            if (isfinite(cert)) atomicAdd((float*)((char*)gm + at), wt[t] * r);
+                            else cert = 0.f;
+                        }
+                        G[t < 13 ? t : 24 - t] = fmaf(cert, r, G[t < 13 ? t : 24 - t]);
+                    }
+                }
+            }
+            float gk[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int t = 0; t < 13; t++) {
+                const int px = t % 5 - 2, py = t / 5 - 2;
+                if (!live[t]) continue;
+                const float gw = G[t] * wt[t];
+                gk[0] += -0.5f * (float)(px * px) * gw;
+                gk[1] += -0.5f * (float)(py * py) * gw;
+                gk[2] += -(float)(px * py) * gw;
+            }
+            kparam_scatter(gkp, g.W, g.H, xb, yb, gk);
+        }
+    }
+    loss_sum(lsum, loss);
+}
+
+template <int KC>
+__global__ void __launch_bounds__(256, 2) k_accumulate_bwd_bil(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
                                                        size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* __restrict__ kparam,
                                                        size_t kp_pitch, F3 white, F3 black, const float* __restrict__ out, size_t out_pitch,
                                                        const float* __restrict__ wsum, size_t ws_pitch, const float* __restrict__ target,
@@ -348,100 +566,64 @@ __global__ void __launch_bounds__(256, 2) k_accumulate_bwd(isa_accum_geom g, uns
                 float bx = 0.f, by = 0.f;
                 if (fr.flow) {
                     float2 fl = flow_sample(fr.flow, flow_pitch, g.W, g.H, xb, yb);
-                    if constexpr (BIL) {
-                        const float hx = fl.x * g.s, hy = fl.y * g.s;
-                        const float fx = floorf(hx), fy = floorf(hy);
-                        sx0 = (int)fx; sy0 = (int)fy;
-                        bx = hx - fx; by = hy - fy;
-                    } else {
-                        sx0 = (int)roundf(fl.x * g.s);
-                        sy0 = (int)roundf(fl.y * g.s);
-                    }
+                    const float hx = fl.x * g.s, hy = fl.y * g.s;
+                    const float fx = floorf(hx), fy = floorf(hy);
+                    sx0 = (int)fx; sy0 = (int)fy;
+                    bx = hx - fx; by = hy - fy;
                 }
                 float4* gm = gmask + (size_t)f * gmask_stride;
                 float D[4] = {0.f, 0.f, 0.f, 0.f};
-                if constexpr (BIL) {
-                    // taps outer, corners inner (as the forward): the 6 x 6 positions once, the tap's mask cell and
-                    // its gradient (per channel, summed over the corners) once per tap
-                    const float wk[4] = {(1.f - bx) * (1.f - by), bx * (1.f - by), (1.f - bx) * by, bx * by};
-                    const bool need_d = fr.flow != nullptr;
-                    int qxs[6], qys[6];
-                    const uint16_t* rrs[6];
+                // taps outer, corners inner (as the forward): the 6 x 6 positions once, the tap's mask cell and
+                // its gradient (per channel, summed over the corners) once per tap
+                const float wk[4] = {(1.f - bx) * (1.f - by), bx * (1.f - by), (1.f - bx) * by, bx * by};
+                const bool need_d = fr.flow != nullptr;
+                int qxs[6], qys[6];
+                const uint16_t* rrs[6];
 #pragma unroll
-                    for (int d = 0; d < 6; d++) {
-                        qxs[d] = isa::clampi(floor_div_s(x + d - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
-                        qys[d] = isa::clampi(floor_div_s(y + d - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
-                        rrs[d] = isa::row_ptr(fr.raw, raw_pitch, qys[d]);
-                    }
+                for (int d = 0; d < 6; d++) {
+                    qxs[d] = isa::clampi(floor_div_s(x + d - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
+                    qys[d] = isa::clampi(floor_div_s(y + d - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
+                    rrs[d] = isa::row_ptr(fr.raw, raw_pitch, qys[d]);
+                }
 #pragma unroll
-                    for (int py = 0; py < 5; py++) {
-                        const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
+                for (int py = 0; py < 5; py++) {
+                    const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
 #pragma unroll
-                        for (int px = 0; px < 5; px++) {
-                            float4 m = make_float4(1.f, 1.f, 1.f, 1.f);
-                            if (mr) m = __ldg(mr + ux[px]);
-                            const float ww = wt[py * 5 + px];
-                            float gc[3] = {0.f, 0.f, 0.f}, Gt = 0.f;
+                    for (int px = 0; px < 5; px++) {
+                        float4 m = make_float4(1.f, 1.f, 1.f, 1.f);
+                        if (mr) m = __ldg(mr + ux[px]);
+                        const float ww = wt[py * 5 + px];
+                        float gc[3] = {0.f, 0.f, 0.f}, Gt = 0.f;
 #pragma unroll
-                            for (int corner = 0; corner < 4; corner++) {
-                                if (wk[corner] == 0.f && !need_d) continue;
-                                const int dx = corner & 1, dy = corner >> 1;
-                                const int qx = qxs[px + dx], qy = qys[py + dy];
-                                const int c = isa::cfa_at(cfa, qx, qy);
-                                if (c > 2) continue;
-                                float raw = (float)__ldg(rrs[py + dy] + qx);
-                                raw = (raw - black.v[c]) / white.v[c];
-                                const float hc = c == 0 ? h[0] : (c == 1 ? h[1] : h[2]);
-                                const float oc = c == 0 ? o[0] : (c == 1 ? o[1] : o[2]);
-                                const float r = hc * (raw - oc);
-                                float cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
-                                if (!isfinite(cert)) cert = 0.f;
-                                else if (c == 0) gc[0] += ww * r * wk[corner];
-                                else if (c == 1) gc[1] += ww * r * wk[corner];
-                                else gc[2] += ww * r * wk[corner];
-                                D[corner] += ww * cert * r;
-                                Gt += cert * r * wk[corner];
-                            }
-                            G[py * 5 + px] += Gt;
-                            if (mr) {
-                                float* dst = (float*)(isa::row_ptr(gm, mask_pitch, uy[py]) + ux[px]);
-#pragma unroll
-                                for (int c = 0; c < 3; c++)
-                                    if (gc[c] != 0.f) atomicAdd(dst + c, gc[c]);
-                            }
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int py = 0; py < 5; py++) {
-                        const int qy = isa::clampi(floor_div_s(y + py - 2 + sy0 + g.oy, g), g.cy0, g.cy1);
-                        const uint16_t* rr = isa::row_ptr(fr.raw, raw_pitch, qy);
-                        const float4* mr = fr.mask ? isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
-#pragma unroll
-                        for (int px = 0; px < 5; px++) {
-                            const int qx = isa::clampi(floor_div_s(x + px - 2 + sx0 + g.ox, g), g.cx0, g.cx1);
+                        for (int corner = 0; corner < 4; corner++) {
+                            if (wk[corner] == 0.f && !need_d) continue;
+                            const int dx = corner & 1, dy = corner >> 1;
+                            const int qx = qxs[px + dx], qy = qys[py + dy];
                             const int c = isa::cfa_at(cfa, qx, qy);
                             if (c > 2) continue;
-                            float raw = (float)__ldg(rr + qx);
+                            float raw = (float)__ldg(rrs[py + dy] + qx);
                             raw = (raw - black.v[c]) / white.v[c];
                             const float hc = c == 0 ? h[0] : (c == 1 ? h[1] : h[2]);
                             const float oc = c == 0 ? o[0] : (c == 1 ? o[1] : o[2]);
                             const float r = hc * (raw - oc);
-                            float cert = 1.f;
-                            if (mr) {
-                                const float4 m = __ldg(mr + ux[px]);
-                                cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
-                                if (!isfinite(cert)) cert = 0.f;
-                                else {
-                                    float* dst = (float*)(isa::row_ptr(gm, mask_pitch, uy[py]) + ux[px]) + c;
-                                    atomicAdd(dst, wt[py * 5 + px] * r);
-                                }
-                            }
-                            G[py * 5 + px] += cert * r;
+                            float cert = c == 0 ? m.x : (c == 1 ? m.y : m.z);
+                            if (!isfinite(cert)) cert = 0.f;
+                            else if (c == 0) gc[0] += ww * r * wk[corner];
+                            else if (c == 1) gc[1] += ww * r * wk[corner];
+                            else gc[2] += ww * r * wk[corner];
+                            D[corner] += ww * cert * r;
+                            Gt += cert * r * wk[corner];
+                        }
+                        G[py * 5 + px] += Gt;
+                        if (mr) {
+                            float* dst = (float*)(isa::row_ptr(gm, mask_pitch, uy[py]) + ux[px]);
+#pragma unroll
+                            for (int c = 0; c < 3; c++)
+                                if (gc[c] != 0.f) atomicAdd(dst + c, gc[c]);
                         }
                     }
                 }
-                if (BIL && fr.flow && gflow) {
+                if (fr.flow && gflow) {
                     const float dbx = (1.f - by) * (D[1] - D[0]) + by * (D[3] - D[2]);
                     const float dby = (1.f - bx) * (D[2] - D[0]) + bx * (D[3] - D[1]);
                     flow_scatter(gflow, flow_pitch, g.W, g.H, xb, yb, dbx * g.s, dby * g.s);
@@ -460,31 +642,10 @@ __global__ void __launch_bounds__(256, 2) k_accumulate_bwd(isa_accum_geom g, uns
                     gk[1] += -0.5f * (float)(py * py) * gw;
                     gk[2] += -(float)(px * py) * gw;
                 }
-            const float fx = floorf(xb), fy = floorf(yb);
-            const int i = (int)fx, j = (int)fy;
-            const float a = xb - fx, b = yb - fy;
-            const int i0 = isa::clampi(i, 0, g.W - 1), i1 = isa::clampi(i + 1, 0, g.W - 1), j0 = isa::clampi(j, 0, g.H - 1), j1 = isa::clampi(j + 1, 0, g.H - 1);
-            const float w00 = (1.f - a) * (1.f - b), w10 = a * (1.f - b), w01 = (1.f - a) * b, w11 = a * b;
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                atomicAdd(gkp + ((size_t)j0 * g.W + i0) * 3 + c, w00 * gk[c]);
-                if (a != 0.f) atomicAdd(gkp + ((size_t)j0 * g.W + i1) * 3 + c, w10 * gk[c]);
-                if (b != 0.f) atomicAdd(gkp + ((size_t)j1 * g.W + i0) * 3 + c, w01 * gk[c]);
-                if (a != 0.f && b != 0.f) atomicAdd(gkp + ((size_t)j1 * g.W + i1) * 3 + c, w11 * gk[c]);
-            }
+            kparam_scatter(gkp, g.W, g.H, xb, yb, gk);
         }
     }
-    // block sum of the loss, one atomic per block
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    __shared__ double sl[8];
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    if ((tid & 31) == 0) sl[tid >> 5] = lsum;
-    __syncthreads();
-    if (tid == 0 && loss) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x * blockDim.y) / 32; w++) t += sl[w];
-        atomicAdd(loss, t);
-    }
+    loss_sum(lsum, loss);
 }
 
 // dL/d(kDetail, kDenoise, Dth, Dtr, kStretch, kShrink) from dL/dkparam: the
@@ -583,27 +744,20 @@ cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const i
         return isa_launch_accumulate_bayer(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc, wsum,
                                         out_pitch, accumulate_into, st);
     if (nframes > 1 && !frames_dev) return cudaErrorInvalidValue;
-    F3 wh, bl;
-    for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; bl.v[c] = black[c]; }
+    F3 wh, rw, bl;
+    for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; rw.v[c] = (float)(1.0 / (double)white[c]); bl.v[c] = black[c]; }
     const isa_frame_in one = nframes == 1 ? frames[0] : isa_frame_in{nullptr, nullptr, nullptr};
     const isa_frame_in* list = nframes == 1 ? nullptr : frames_dev;
     if (g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
     dim3 b(g.bx > 0 ? g.bx : 32, g.by > 0 ? g.by : 8), grd = grid2(g.Wo, g.yb1 - g.yb0, b);
     if (b.x * b.y > 256) return cudaErrorInvalidValue;
-    if (kparam_channels == 4 && g.bilinear)
-        k_accumulate<4, true><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
-                                                 wsum, out_pitch, accumulate_into);
-    else if (kparam_channels == 4)
-        k_accumulate<4, false><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
-                                                  wsum, out_pitch, accumulate_into);
-    else if (kparam_channels == 3 && g.bilinear)
-        k_accumulate<3, true><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
-                                                 wsum, out_pitch, accumulate_into);
-    else if (kparam_channels == 3)
-        k_accumulate<3, false><<<grd, b, 0, st>>>(g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc,
-                                                  wsum, out_pitch, accumulate_into);
+    if (kparam_channels != 3 && kparam_channels != 4) return cudaErrorInvalidValue;
+    if (g.bilinear)
+        (kparam_channels == 4 ? k_accumulate_bil<4> : k_accumulate_bil<3>)<<<grd, b, 0, st>>>(
+            g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc, wsum, out_pitch, accumulate_into);
     else
-        return cudaErrorInvalidValue;
+        (kparam_channels == 4 ? k_accumulate<4> : k_accumulate<3>)<<<grd, b, 0, st>>>(
+            g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, rw, bl, acc, wsum, out_pitch, accumulate_into);
     return cudaGetLastError();
 }
 
@@ -625,13 +779,11 @@ cudaError_t isa_launch_accumulate_bwd(const isa_accum_geom& g, unsigned cfa, con
     for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; bl.v[c] = black[c]; }
     dim3 b(32, 8), grd = grid2(g.Wo, g.Ho, b);
     if (g.bilinear)
-        k_accumulate_bwd<4, true><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out,
-                                                     out_pitch, wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss,
-                                                     gflow);
+        k_accumulate_bwd_bil<4><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out,
+                                                   out_pitch, wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss, gflow);
     else
-        k_accumulate_bwd<4, false><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out,
-                                                      out_pitch, wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss,
-                                                      nullptr);
+        k_accumulate_bwd<4><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out, out_pitch,
+                                               wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss);
     return cudaGetLastError();
 }
 
