@@ -13,6 +13,7 @@
 #include "isa_internal.cuh"
 #include <float.h>
 #include <algorithm>
+#include <type_traits>
 
 namespace {
 
@@ -54,6 +55,81 @@ struct TrackDims {
     static constexpr int TOTAL = OFF_MAP + D * D;
     static constexpr size_t BYTES = (size_t)TOTAL * sizeof(float);
 };
+
+// findMinimum (kernel.cu:422-546) over a tile's L2 map in shared memory and preShift += result (:355-358), by one warp. tix:
+// the tile's place in the outputs; pre: the pre-shift at *grid.
+template <int D, int S>
+__device__ __forceinline__ void track_result(const float* map, int lane, size_t tix, int oxt, int oyt, float2 pre, float2* grid, float threshold,
+                                             float* __restrict__ scores, int* __restrict__ argmin_out, int* __restrict__ offsets_out)
+{
+    // first strict minimum and maximum over the map
+    float mn = FLT_MAX, mx = -FLT_MAX;
+    int mi = 0x7fffffff;
+    for (int i = lane; i < D * D; i += 32) {
+        const float v = map[i];
+        mx = fmaxf(mx, v);
+        if (v < mn) { mn = v; mi = i; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float omn = __shfl_xor_sync(0xffffffffu, mn, o), omx = __shfl_xor_sync(0xffffffffu, mx, o);
+        const int omi = __shfl_xor_sync(0xffffffffu, mi, o);
+        if (omn < mn || (omn == mn && omi < mi)) { mn = omn; mi = omi; }
+        mx = fmaxf(mx, omx);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        if (mi == 0x7fffffff) mi = -1;
+        if (argmin_out) argmin_out[tix] = mi;
+        if (offsets_out) { offsets_out[2 * tix] = oxt; offsets_out[2 * tix + 1] = oyt; }
+        float cx = 0.f, cy = 0.f;
+        if (mi >= 0) {
+            int iy = mi / D, ix = mi - iy * D;
+            cy = (float)iy;
+            cx = (float)ix;
+            if (ix < 1 || iy < 1 || ix >= 2 * S || iy >= 2 * S) {
+                cx = 0.f; cy = 0.f;
+            } else {
+                float a11 = 0.f, a22 = 0.f, a12 = 0.f, b1 = 0.f, b2 = 0.f;
+#pragma unroll
+                for (int k = 0; k < 9; k++) {
+                    float v = map[(iy + k / 3 - 1) * D + ix + k % 3 - 1];
+                    a11 += c_fit[0][k] * v; a22 += c_fit[1][k] * v; a12 += c_fit[2][k] * v;
+                    b1 += c_fit[3][k] * v; b2 += c_fit[4][k] * v;
+                }
+                a11 = fmaxf(a11, 0.0f);
+                a22 = fmaxf(a22, 0.0f);
+                float det = a11 * a22 - a12 * a12;
+                if (det < 0) { a12 = 0; det = a11 * a22; }
+                if (det != 0) {
+                    float mux = (a22 * b1 - a12 * b2) / det, muy = (a11 * b2 - a12 * b1) / det;
+                    if (fabsf(mux) > 1) mux = 0;
+                    if (fabsf(muy) > 1) muy = 0;
+                    cx -= mux; cy -= muy;
+                }
+                cx -= S; cy -= S;
+            }
+        }
+        if (threshold + mn > mx) { cx = 0.f; cy = 0.f; }
+        pre.x += cx;
+        pre.y += cy;
+        *grid = pre;
+    }
+    if (scores) {
+        __syncwarp();
+        for (int i = lane; i < D * D; i += 32) scores[tix * D * D + i] = map[i];
+    }
+}
+
+// f(0), f(1), ..., f(N - 1) with compile-time arguments.
+template <int N, int I = 0, class F>
+__device__ __forceinline__ void unroll(F&& f)
+{
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        unroll<N, I + 1>(f);
+    }
+}
 
 // Thread (row pair, sy) streams template rows 2i, 2i + 1 against block rows
 // 2i + sy, 2i + 1 + sy with a D-wide register window of float2 pairs,
@@ -196,67 +272,8 @@ __global__ void __launch_bounds__(TrackDims<T, S>::NT) k_track(const float* cons
         for (int k = 0; k < D; k++) map[sy * D + k] = sum[k];
     }
     __syncthreads();
-    if (warp == 0) {
-        // map = sum of the partials; first strict minimum and maximum over the map
-        float mn = FLT_MAX, mx = -FLT_MAX;
-        int mi = 0x7fffffff;
-        for (int i = lane; i < D * D; i += 32) {
-            const float v = map[i];
-            mx = fmaxf(mx, v);
-            if (v < mn) { mn = v; mi = i; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float omn = __shfl_xor_sync(0xffffffffu, mn, o), omx = __shfl_xor_sync(0xffffffffu, mx, o);
-            const int omi = __shfl_xor_sync(0xffffffffu, mi, o);
-            if (omn < mn || (omn == mn && omi < mi)) { mn = omn; mi = omi; }
-            mx = fmaxf(mx, omx);
-        }
-        __syncwarp();
-        if (lane == 0) {
-            if (mi == 0x7fffffff) mi = -1;
-            size_t tix = (size_t)p * tcx * tcy + tile;
-            if (argmin_out) argmin_out[tix] = mi;
-            if (offsets_out) { offsets_out[2 * tix] = oxt; offsets_out[2 * tix + 1] = oyt; }
-            float cx = 0.f, cy = 0.f;
-            if (mi >= 0) {
-                int iy = mi / D, ix = mi - iy * D;
-                cy = (float)iy;
-                cx = (float)ix;
-                if (ix < 1 || iy < 1 || ix >= 2 * S || iy >= 2 * S) {
-                    cx = 0.f; cy = 0.f;
-                } else {
-                    float a11 = 0.f, a22 = 0.f, a12 = 0.f, b1 = 0.f, b2 = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 9; k++) {
-                        float v = map[(iy + k / 3 - 1) * D + ix + k % 3 - 1];
-                        a11 += c_fit[0][k] * v; a22 += c_fit[1][k] * v; a12 += c_fit[2][k] * v;
-                        b1 += c_fit[3][k] * v; b2 += c_fit[4][k] * v;
-                    }
-                    a11 = fmaxf(a11, 0.0f);
-                    a22 = fmaxf(a22, 0.0f);
-                    float det = a11 * a22 - a12 * a12;
-                    if (det < 0) { a12 = 0; det = a11 * a22; }
-                    if (det != 0) {
-                        float mux = (a22 * b1 - a12 * b2) / det, muy = (a11 * b2 - a12 * b1) / det;
-                        if (fabsf(mux) > 1) mux = 0;
-                        if (fabsf(muy) > 1) muy = 0;
-                        cx -= mux; cy -= muy;
-                    }
-                    cx -= S; cy -= S;
-                }
-            }
-            if (threshold + mn > mx) { cx = 0.f; cy = 0.f; }
-            pre.x += cx;
-            pre.y += cy;
-            gline[tx] = pre;
-        }
-        if (scores) {
-            __syncwarp();
-            const size_t tix = (size_t)p * tcx * tcy + tile;
-            for (int i = lane; i < D * D; i += 32) scores[tix * D * D + i] = map[i];
-        }
-    }
+    if (warp == 0)
+        track_result<D, S>(map, lane, (size_t)p * tcx * tcy + tile, oxt, oyt, pre, gline + tx, threshold, scores, argmin_out, offsets_out);
 }
 
 template <int T, int S>
@@ -271,6 +288,275 @@ cudaError_t launch_track_ts(const float* const* frames, size_t pitch, int Wl, in
     }
     dim3 g(npairs, tcx * tcy);
     k_track<T, S><<<g, L::NT, L::BYTES, st>>>(frames, pitch, Wl, Hl, tcx, tcy, pairs, grids, grid_pitch, grid_stride, thr, scores, argmin, offsets);
+    return cudaGetLastError();
+}
+
+// ---- one warp per (frame pair, tile) --------------------------------------------
+// For tiles of 32 and 16 rows in large searches. A lane owns a template row
+// (and, for the smaller tiles, a 1 / G share of the shift rows): per column it loads one
+// template value and one value of each block row it needs, keeps the last D
+// values of each row in registers and adds (r - t)^2 to all its (shift row,
+// column shift) sums, two shift rows in the two halves of packed FP32x2
+// arithmetic. Each sum runs over its row's columns in order, then the two rows
+// of a pair are added, then the pairs across lanes: the additions and their
+// order are k_track's, so are the results, bit for bit.
+// A warp works through a run of pairs of one tile: the block of the next pair
+// (and its template, when the reference changes) comes in by cp.async while
+// the current one is searched, and the descriptor after that is on its way in
+// registers, so the chain pair table -> pre-shift -> frame table -> tile loads
+// is off the critical path.
+// Bound: the FMA pipe (2 lane operations per template pixel and shift), busy
+// about 60 %; 12 warps per SM (15 KB of shared memory each) leave the chains of
+// staging and minimum search partly exposed. All 190 pairs of 20 x 6016x4000:
+// tile alignment (four levels and solves) 29.1 -> 23.0 ms.
+template <int T, int S>
+struct WarpDims {
+    static_assert(T <= 32 && 32 % T == 0, "rows of a tile are lanes");
+    static constexpr int B = T + 2 * S, D = 2 * S + 1;
+    static constexpr int G = 32 / T;                 // lane groups, each with its share of the shift rows
+    static constexpr int NSY = (D + G - 1) / G;      // shift rows per group
+    static constexpr int SP0 = 27 / D < 1 ? 1 : 27 / D;
+    static constexpr int SP = SP0 < NSY ? SP0 : NSY; // shift rows per pass: up to 27 running sums in registers
+    static constexpr int NP = (NSY + SP - 1) / SP;   // passes
+    static constexpr bool EXACT = G * NP * SP == D;  // no shift row beyond the last
+    static constexpr int TP = T + 1, BP = B + 1;     // odd strides: conflict-free column reads
+    static constexpr int BLK = (B * BP + 3) / 4 * 4;
+    static constexpr int OFF_BLK = (T * TP + 3) / 4 * 4, OFF_MAP = OFF_BLK + 2 * BLK;
+    static constexpr int FLOATS = OFF_MAP + (D * D + 3) / 4 * 4;
+    static constexpr int WARPS = 4;
+    static constexpr size_t BYTES = (size_t)FLOATS * WARPS * sizeof(float);
+};
+
+// Sums of v[0 .. N) over the lanes, distributed: on return lane l holds in v[0] the total of entry idx (returned, N or more:
+// none). Lanes are combined in the order of the masks 1, 16, 8, 4, 2 (M: the masks left to do), halving the entries a
+// lane carries on each step.
+template <int N, int M>
+__device__ __forceinline__ int lane_sums(float (&v)[N], int lane)
+{
+    constexpr int NEXT = M == 1 ? 16 : M >> 1;
+    constexpr int HALF = (N + 1) / 2;
+    const bool up = lane & M;
+    float u[HALF];
+#pragma unroll
+    for (int i = 0; i < HALF; i++) {
+        const float lo = v[i], hi = i + HALF < N ? v[i + HALF] : 0.f;
+        u[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, M);
+    }
+    int at = 0;
+    if constexpr (M != 2) {
+        at = lane_sums<HALF, NEXT>(u, lane);
+    } else {
+        static_assert(HALF == 1, "one entry per lane at the end");
+    }
+    v[0] = u[0];
+    return (at >= HALF ? N : at) + (up ? HALF : 0);
+}
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// N x N pixels at (x0, y0) of a level image into shared memory (row stride P), with replicate borders.
+template <int N, int P>
+__device__ __forceinline__ void stage_tile(float* dst, const float* img, size_t pitch, int Wl, int Hl, int x0, int y0, int lane)
+{
+    constexpr int C = N < 32 ? N : 32, REST = N - C;  // columns by lane, and the rest several rows at a time
+    constexpr int RQ = 32 / C, RR = REST > 0 ? 32 / (REST > 0 ? REST : 1) : 1;  // rows per step of either part
+    const int c1 = lane % C, r1 = lane / C, c2 = REST > 0 ? C + lane % (REST > 0 ? REST : 1) : 0, r2 = REST > 0 ? lane / (REST > 0 ? REST : 1) : 0;
+    float* d1 = dst + r1 * P + c1;
+    float* d2 = dst + r2 * P + c2;
+    if (x0 >= 0 && y0 >= 0 && x0 + N <= Wl && y0 + N <= Hl) {
+        const float* p1 = isa::row_ptr(img, pitch, y0 + r1) + x0 + c1;
+#pragma unroll
+        for (int i = 0; i < (N + RQ - 1) / RQ; i++) {
+            if (r1 < RQ && (N % RQ == 0 || i * RQ + r1 < N)) cp_async4(d1 + i * RQ * P, p1);
+            p1 = isa::row_ptr(p1, pitch, RQ);
+        }
+        if constexpr (REST > 0) {
+            const float* p2 = isa::row_ptr(img, pitch, y0 + r2) + x0 + c2;
+#pragma unroll
+            for (int i = 0; i < (N + RR - 1) / RR; i++) {
+                if (r2 < RR && i * RR + r2 < N) cp_async4(d2 + i * RR * P, p2);
+                p2 = isa::row_ptr(p2, pitch, RR);
+            }
+        }
+    } else {
+        const float* p1 = img + isa::clampi(x0 + c1, 0, Wl - 1);
+#pragma unroll 1
+        for (int i = 0; i < (N + RQ - 1) / RQ; i++)
+            if (r1 < RQ && i * RQ + r1 < N) cp_async4(d1 + i * RQ * P, isa::row_ptr(p1, pitch, isa::clampi(y0 + i * RQ + r1, 0, Hl - 1)));
+        if constexpr (REST > 0) {
+            const float* p2 = img + isa::clampi(x0 + c2, 0, Wl - 1);
+#pragma unroll 1
+            for (int i = 0; i < (N + RR - 1) / RR; i++)
+                if (r2 < RR && i * RR + r2 < N) cp_async4(d2 + i * RR * P, isa::row_ptr(p2, pitch, isa::clampi(y0 + i * RR + r2, 0, Hl - 1)));
+        }
+    }
+}
+
+// A pair's place in the search: template and block origins, block image, pre-shift and its grid entry.
+struct WarpItem {
+    const float *ref, *trk;
+    float2* grid;
+    float2 pre;
+    int xr, yr, xt, yt;  // template and block origins
+    int oxt, oyt;        // the block's integer offset
+};
+
+template <int T, int S>
+__device__ __forceinline__ WarpItem warp_item(const float* const* frames, const isa_pair_desc* pairs, int p, int tx, int ty, int Wl, int Hl, float2* grids,
+                                              size_t grid_pitch, size_t grid_stride)
+{
+    const isa_pair_desc pd = pairs[p];
+    WarpItem it;
+    it.grid = (float2*)((char*)grids + (size_t)pd.grid * grid_stride + (size_t)ty * grid_pitch) + tx;
+    it.pre = *it.grid;
+    it.ref = frames[pd.ref];
+    it.trk = frames[pd.trk];
+    int oxr, oyr;
+    tile_offset(tx, ty, T, Wl, Hl, pd.base_ref_x, pd.base_ref_y, pd.rot_ref, 0.f, 0.f, oxr, oyr);
+    tile_offset(tx, ty, T, Wl, Hl, pd.base_trk_x, pd.base_trk_y, pd.rot_trk, it.pre.x, it.pre.y, it.oxt, it.oyt);
+    it.xr = tx * T + S + oxr; it.yr = ty * T + S + oyr;
+    it.xt = tx * T + it.oxt; it.yt = ty * T + it.oyt;
+    return it;
+}
+
+template <int T, int S>
+__global__ void __launch_bounds__(32 * WarpDims<T, S>::WARPS, 3) k_track_warp(const float* const* __restrict__ frames, size_t pitch, int Wl, int Hl, int tcx,
+                                                                            int ntiles, const isa_pair_desc* __restrict__ pairs, int npairs, int run,
+                                                                            int nruns, float2* __restrict__ grids, size_t grid_pitch, size_t grid_stride,
+                                                                            float threshold, float* __restrict__ scores, int* __restrict__ argmin_out,
+                                                                            int* __restrict__ offsets_out)
+{
+    using L = WarpDims<T, S>;
+    constexpr int B = L::B, D = L::D, SP = L::SP, NSY = L::NSY, BP = L::BP, TP = L::TP;
+    extern __shared__ __align__(16) float smf[];
+    const int lane = threadIdx.x & 31;
+    const int w = blockIdx.x * L::WARPS + (threadIdx.x >> 5);
+    const int tile = w / nruns, p0 = (w - tile * nruns) * run, p1 = min(p0 + run, npairs);
+    if (tile >= ntiles) return;  // the whole warp leaves; only warp-level synchronisation below
+    float* tpl = smf + (threadIdx.x >> 5) * L::FLOATS;
+    float* map = tpl + L::OFF_MAP;
+    const int ty = tile / tcx, tx = tile - ty * tcx;
+    const int y = lane % T, grp = lane / T;
+    WarpItem cur = warp_item<T, S>(frames, pairs, p0, tx, ty, Wl, Hl, grids, grid_pitch, grid_stride);
+    stage_tile<T, TP>(tpl, cur.ref, pitch, Wl, Hl, cur.xr, cur.yr, lane);
+    stage_tile<B, BP>(tpl + L::OFF_BLK, cur.trk, pitch, Wl, Hl, cur.xt, cur.yt, lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    WarpItem next = warp_item<T, S>(frames, pairs, min(p0 + 1, p1 - 1), tx, ty, Wl, Hl, grids, grid_pitch, grid_stride);
+#pragma unroll 1
+    for (int p = p0; p < p1; p++) {
+        const float* blk = tpl + L::OFF_BLK + ((p - p0) & 1) * L::BLK;
+        // the next pair's block into the other buffer; its last reader was the search before this one (the warp has
+        // synchronised since)
+        if (p + 1 < p1) stage_tile<B, BP>(tpl + L::OFF_BLK + ((p + 1 - p0) & 1) * L::BLK, next.trk, pitch, Wl, Hl, next.xt, next.yt, lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const WarpItem after = warp_item<T, S>(frames, pairs, min(p + 2, p1 - 1), tx, ty, Wl, Hl, grids, grid_pitch, grid_stride);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+#pragma unroll 1
+        for (int pass = 0; pass < L::NP; pass++) {
+            // this lane's shift rows of the pass (beyond the last: repeated, their sums dropped)
+            const int s0 = grp * NSY + pass * SP;
+            const float* row[SP];
+#pragma unroll
+            for (int j = 0; j < SP; j++) row[j] = L::EXACT ? blk + (y + s0) * BP + j * BP : blk + (y + min(s0 + j, D - 1)) * BP;
+            const float* tr = tpl + y * TP;
+            constexpr int H = SP / 2;  // packed row pairs; an odd row is left
+            float2 acc2[H > 0 ? H : 1][D], win2[H > 0 ? H : 1][D];
+            float acc1[D], win1[D];
+#pragma unroll
+            for (int k = 0; k < D; k++) {
+#pragma unroll
+                for (int j = 0; j < H; j++) acc2[j][k] = make_float2(0.f, 0.f);
+                acc1[k] = 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < D - 1; k++) {
+#pragma unroll
+                for (int j = 0; j < H; j++) win2[j][k] = make_float2(row[2 * j][k], row[2 * j + 1][k]);
+                if constexpr (SP & 1) win1[k] = row[SP - 1][k];
+            }
+            // column x: the newest block value goes to window slot (x + D - 1) % D, shift k reads slot (x + k) % D
+            const auto column = [&](int x, auto ii) {
+                constexpr int i = decltype(ii)::value;
+                constexpr int n = (i + D - 1) % D;
+#pragma unroll
+                for (int j = 0; j < H; j++) win2[j][n] = make_float2(row[2 * j][x + D - 1], row[2 * j + 1][x + D - 1]);
+                if constexpr (SP & 1) win1[n] = row[SP - 1][x + D - 1];
+                const float r = tr[x];
+                const float2 m1 = make_float2(-1.f, -1.f), rr = make_float2(r, r);
+#pragma unroll
+                for (int k = 0; k < D; k++) {
+                    const int q = (i + k) % D;
+#pragma unroll
+                    for (int j = 0; j < H; j++) {
+                        const float2 d = __ffma2_rn(win2[j][q], m1, rr);  // r - t, exactly rounded
+                        acc2[j][k] = __ffma2_rn(d, d, acc2[j][k]);
+                    }
+                    if constexpr (SP & 1) {
+                        const float d = __fsub_rn(r, win1[q]);
+                        acc1[k] = __fmaf_rn(d, d, acc1[k]);
+                    }
+                }
+            };
+            constexpr int FULL = T / D * D;
+#pragma unroll 1
+            for (int x = 0; x < FULL; x += D) unroll<D>([&](auto ii) { column(x + decltype(ii)::value, ii); });
+            unroll<T - FULL>([&](auto ii) { column(FULL + decltype(ii)::value, ii); });
+            // rows of a pair, then the pairs, across lanes; entries (j, k) of the pass
+            if constexpr (L::G == 1) {
+                float v[SP * D];
+#pragma unroll
+                for (int j = 0; j < SP; j++)
+#pragma unroll
+                    for (int k = 0; k < D; k++) v[j * D + k] = (SP & 1) && j == SP - 1 ? acc1[k] : ((j & 1) ? acc2[j / 2][k].y : acc2[j / 2][k].x);
+                const int e = lane_sums<SP * D, 1>(v, lane);
+                if (e < SP * D && pass * SP + e / D < NSY) map[pass * SP * D + e] = v[0];
+            } else {
+#pragma unroll
+                for (int j = 0; j < SP; j++)
+#pragma unroll
+                    for (int k = 0; k < D; k++) {
+                        float v = (SP & 1) && j == SP - 1 ? acc1[k] : ((j & 1) ? acc2[j / 2][k].y : acc2[j / 2][k].x);
+                        v += __shfl_xor_sync(0xffffffffu, v, 1);
+#pragma unroll
+                        for (int o = T / 2; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                        if (y == 0 && pass * SP + j < NSY && s0 + j < D) map[(s0 + j) * D + k] = v;
+                    }
+            }
+        }
+        __syncwarp();
+        // the next reference's template: no lane reads this one any more
+        const bool swap = p + 1 < p1 && (next.ref != cur.ref || next.xr != cur.xr || next.yr != cur.yr);
+        if (swap) {
+            stage_tile<T, TP>(tpl, next.ref, pitch, Wl, Hl, next.xr, next.yr, lane);
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        }
+        track_result<D, S>(map, lane, (size_t)p * ntiles + tile, cur.oxt, cur.oyt, cur.pre, cur.grid, threshold, scores, argmin_out, offsets_out);
+        __syncwarp();
+        cur = next;
+        next = after;
+    }
+}
+
+template <int T, int S>
+cudaError_t launch_track_warp(const float* const* frames, size_t pitch, int Wl, int Hl, int tcx, int tcy, const isa_pair_desc* pairs, int npairs,
+                              float2* grids, size_t grid_pitch, size_t grid_stride, float thr, float* scores, int* argmin, int* offsets, cudaStream_t st)
+{
+    using L = WarpDims<T, S>;
+    cudaError_t e = cudaFuncSetAttribute(k_track_warp<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
+    if (e != cudaSuccess) return e;
+    // pairs per warp: up to 16 (the start of a run is not overlapped), fewer while the runs would not fill the device's
+    // 148 x 12 resident warps eight times over; the runs of a tile about equally long
+    const long long items = (long long)npairs * tcx * tcy;
+    const int most = (int)std::max<long long>(1, std::min<long long>({16, npairs, items / (148 * 12 * 8)}));
+    const int nruns = (npairs + most - 1) / most, run = (npairs + nruns - 1) / nruns;
+    const long long warps = (long long)nruns * tcx * tcy, blocks = (warps + L::WARPS - 1) / L::WARPS;
+    if (warps > 0x7fffffffLL) return cudaErrorInvalidValue;
+    k_track_warp<T, S><<<(unsigned)blocks, 32 * L::WARPS, L::BYTES, st>>>(frames, pitch, Wl, Hl, tcx, tcx * tcy, pairs, npairs, run, nruns, grids, grid_pitch,
+                                                                        grid_stride, thr, scores, argmin, offsets);
     return cudaGetLastError();
 }
 
@@ -496,19 +782,33 @@ __global__ void k_optimal(const float2* __restrict__ x, int n1, int tcx, int tcy
 
 }  // namespace
 
-#define ISA_TRACK_CASE(TT, SS) \
-    if (T == TT && S == SS) return launch_track_ts<TT, SS>(frames, img_pitch, Wl, Hl, tcx, tcy, pairs, npairs, grids, grid_pitch, grid_stride, threshold, scores, argmin, offsets, st);
+// A warp per (pair, tile) or a CTA: the same sums, so the choice is one of time. Few items leave the device idle with a
+// warp each (300 items of 32 x 32, S = 2: 6.8 us against 5.5 us with a CTA each; 2660: 15.3 against 14.3), many keep it
+// busier (7448: 31.1 against 31.3; 19964: 71 against 74; 82908: 252 against 294; S = 4: 27.0 against 26.7 at 2660, 589
+// against 664 at 82908). For 16 x 16 tiles the warp's fixed work weighs more (S = 2, 31668 items: 57 against 60 us;
+// 11310: 25.8 against 24.5), and at S = 4, where its lane groups share nine shift rows unevenly, 205128 items take 625
+// against 643 us but 82908 take 273 against 262. Other tile sizes: a CTA each.
+#define ISA_TRACK_CASE(TT, SS, FROM)                                                                                                            \
+    if (T == TT && S == SS) {                                                                                                                     \
+        if constexpr ((FROM) > 0)                                                                                                                 \
+            if (items >= (FROM))                                                                                                                  \
+                return launch_track_warp<TT, SS>(frames, img_pitch, Wl, Hl, tcx, tcy, pairs, npairs, grids, grid_pitch, grid_stride, threshold,   \
+                                                 scores, argmin, offsets, st);                                                                   \
+        return launch_track_ts<TT, SS>(frames, img_pitch, Wl, Hl, tcx, tcy, pairs, npairs, grids, grid_pitch, grid_stride, threshold, scores,     \
+                                       argmin, offsets, st);                                                                                     \
+    }
 
 cudaError_t isa_launch_track(const float* const* frames, size_t img_pitch, int Wl, int Hl, int T, int S, int tcx, int tcy,
                              const isa_pair_desc* pairs, int npairs, float2* grids, size_t grid_pitch, size_t grid_stride, float threshold,
                              float* scores, int* argmin, int* offsets, cudaStream_t st)
 {
     if (npairs <= 0 || tcx <= 0 || tcy <= 0) return cudaSuccess;
-    ISA_TRACK_CASE(32, 1) ISA_TRACK_CASE(32, 2) ISA_TRACK_CASE(32, 3) ISA_TRACK_CASE(32, 4)
-    ISA_TRACK_CASE(32, 5) ISA_TRACK_CASE(32, 6)
-    ISA_TRACK_CASE(16, 1) ISA_TRACK_CASE(16, 2) ISA_TRACK_CASE(16, 4) ISA_TRACK_CASE(16, 8)
-    ISA_TRACK_CASE(64, 2)
-    ISA_TRACK_CASE(8, 2) ISA_TRACK_CASE(8, 4)
+    const long long items = (long long)npairs * tcx * tcy;
+    ISA_TRACK_CASE(32, 1, 6000) ISA_TRACK_CASE(32, 2, 6000) ISA_TRACK_CASE(32, 3, 6000) ISA_TRACK_CASE(32, 4, 3000)
+    ISA_TRACK_CASE(32, 5, 3000) ISA_TRACK_CASE(32, 6, 3000)
+    ISA_TRACK_CASE(16, 1, 24000) ISA_TRACK_CASE(16, 2, 24000) ISA_TRACK_CASE(16, 4, 0) ISA_TRACK_CASE(16, 8, 0)
+    ISA_TRACK_CASE(64, 2, 0)
+    ISA_TRACK_CASE(8, 2, 0) ISA_TRACK_CASE(8, 4, 0)
     return cudaErrorInvalidValue;
 }
 
