@@ -9,13 +9,15 @@
 // the integer pixel and the sub-pixel flow part so that FP32 keeps full
 // sub-pixel precision far from the origin.
 //
-// k_lk_stream fuses one reference iteration (warp, Set(0) x3, derivatives,
+// k_lk_warp fuses one reference iteration (warp, Set(0) x3, derivatives,
 // lucasKanadeOptim) for a vertical strip of the image, walking down it row by
 // row: FP32 gradient products, FP64 sliding window sums, and the 2x2
 // pseudo-inverse in FP64.
 #include "isa_internal.cuh"
 
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <type_traits>
 
 namespace {
@@ -105,11 +107,58 @@ __device__ __forceinline__ bool lk_matrix(double a, double b, double d, double m
     return r.ok;
 }
 
-__device__ __forceinline__ float2 lk_update(float2 f, double a, double b, double d, double sxt, double syt, double min_det)
+// Out of line: the per-pixel kernel calls it only where lk_update_n's quick
+// decisions are not certain.
+__device__ __noinline__ float2 lk_update(float2 f, double a, double b, double d, double sxt, double syt, double min_det)
 {
     double m0, m1, m2, m3;
     if (!lk_matrix(a, b, d, min_det, m0, m1, m2, m3)) return f;
     return lk_apply(f, m0, m1, m2, m3, sxt, syt);
+}
+
+// lk_update at the pixels of f (v: the five window sums of each; on: pixels to
+// update). The usual case, a well-conditioned matrix, runs without a branch at
+// all pixels side by side: a branch or a division's own slow path between
+// them would put their FP64 chains one after the other. The largest
+// eigenvalue only steers the two threshold tests; here it is good to 1e-5, so
+// a pixel that close to a threshold goes through lk_update, and so does every
+// pixel with a NaN or a matrix far out of range. 1 / det: an approximate
+// reciprocal x and a third-order step x (1 + e + e^2), e = 1 - det x; neither
+// it nor the square root passes through FP32, whose conversions are the
+// scarcest instructions here.
+template <int N>
+__device__ __forceinline__ void lk_update_n(float2 (&f)[N], const double (&v)[5][N], const bool (&on)[N], double min_det)
+{
+    float2 g[N];
+    bool slow[N], any = false;
+    const double lo = min_det * 0.99999, hi = min_det * 1.00001;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const double a = v[0][k], b = v[1][k], d = v[2][k], sxt = v[3][k], syt = v[4][k];
+        const double hd = 0.5 * (a - d), s = fma(hd, hd, b * b);
+        const double det = fma(a, d, -(b * b));
+        double r, x;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(det));
+        const double l1 = fma(s, r, 0.5 * (a + d));
+        const double e = fma(-det, x, 1.0);
+        const double inv = fma(x, fma(e, e, e), x);
+        const double du = (d * sxt - b * syt) * inv, dv = (a * syt - b * sxt) * inv;
+        const bool well = det > 1.00001e-3 * (l1 * l1) && l1 > 1e-15 && l1 < 1e15;
+        const bool keep = well && l1 < lo;
+        const bool up = well && l1 > hi && fabs(du) < 1e30 && fabs(dv) < 1e30;
+        g[k] = up ? make_float2((float)((double)f[k].x + du), (float)((double)f[k].y + dv)) : f[k];
+        slow[k] = on[k] && !keep && !up;
+        any |= slow[k];
+    }
+    if (any) {
+#pragma unroll
+        for (int k = 0; k < N; k++)
+            if (slow[k]) g[k] = lk_update(f[k], v[0][k], v[1][k], v[2][k], v[3][k], v[4][k], min_det);
+    }
+#pragma unroll
+    for (int k = 0; k < N; k++)
+        if (on[k]) f[k] = g[k];
 }
 
 // Adjoint of lk_update at one pixel for the upstream gradient g of the
@@ -244,44 +293,112 @@ __global__ void k_lk_sums(float2* flow, size_t flow_pitch, const float* __restri
 }
 
 // Streaming form of one reference iteration (warp, Set(0) x3, derivatives,
-// lucasKanadeOptim). A CTA of LKS_NT threads owns a vertical strip of LKS_NT
-// columns (SW = LKS_NT - 2R output columns, R = h + 2) and `sh` output rows:
-// thread t owns image column x0 - R + t (mirrored at the border) and walks
-// down the strip two rows per step:
-//   1. the warped source and the reference of the two rows go into a ring of
-//      six rows of (warped, reference) pairs in shared memory; the global
-//      loads of the next two rows are issued one step ahead (bilinear
-//      samples) and two steps ahead (flow);
-//   2. after a barrier, five-tap derivatives at the two centre rows (own
-//      column and neighbours from the ring), FP32 products, and per-column
-//      vertical window sums in FP64 registers (the product leaving the
-//      window comes from a shared ring of the last 2h + 1 product rows that
-//      only its own thread touches);
-//   3. after a second barrier, the row window sums of the two output rows
-//      (2h + 1 columns, two pixels per thread, FP64) and the 2x2 solve.
+// lucasKanadeOptim). A warp owns a vertical strip of LKW_NC columns (two a
+// lane) and `sh` output rows and walks down it row by row, with no barrier
+// wider than the warp:
+//   1. the warped source and the reference of the row go into a ring of rows
+//      in shared memory (lane l writes columns l and l + 32, so the global
+//      loads and the bilinear taps are coalesced); the taps of the next row
+//      and the flow of the one after are already on their way;
+//   2. lane l reads columns 2l, 2l + 1 back, with two neighbours either side
+//      and the rows above and below: five-tap derivatives at the centre row,
+//      FP32 products, and per-column vertical window sums in FP64 registers.
+//      The products leaving the window are formed again from a ring of the
+//      last 2h + 1 rows of (dx, dy, dt), the same three numbers rounded in the
+//      same way, so what is subtracted is what was added;
+//   3. row window sums in FP64: a lane's outputs are the two windows that
+//      start in its own columns; both hold the lanes between whole, summed
+//      from runs of 1, 2, 4, ... lanes by shuffles (five exchanged values and
+//      eight additions per channel and two pixels at h = 5); then the 2x2
+//      solve. Lane l's outputs lie h columns to the right of its own and leave
+//      as 16-byte stores where rows are aligned.
 // The FP64 sums hold the FP32 products exactly enough that the order of
-// summation does not matter at FP32 output precision. Threads at the strip's
-// edges (t < 2, t >= LKS_NT - 2) compute products from padding; their column
-// sums are never read.
-constexpr int LKS_NT = 128, LKS_PX = 2;
+// summation does not matter at FP32 output precision. Columns at the strip's
+// edges form products from padding; no window reads their sums.
+//
+// Bound by latency and issue (55 % of issue slots at 12 warps an SM, 126 M
+// warp instructions at 4000x3000; FP64 and conversions 26 % and 42 % of their
+// pipes, DRAM 13 %), not by HBM (24 bytes a pixel). Before, a CTA of 128 threads
+// walked a strip of 114 columns two rows a step, behind two barriers a step,
+// and read 240 bytes of column sums a pixel from shared memory for the row
+// sums. One iteration, h = 5, before -> now: 640x480 45 -> 30 us, 1024x768
+// 49 -> 43, 4000x3000 273 -> 227, 6016x4000 500 -> 405. Four columns a lane
+// (half the shuffles, but 250 registers and 8 warps an SM): 42, 47, 234, 417.
+constexpr int LKW_NC = 64;
+constexpr int LKW_WARPS = 4;  // strips (warps) per CTA, one per scheduler of the SM: they share nothing
+constexpr int LKW_CTAS = 3;   // per SM: 168 registers a thread; with 4 the row sums and the solve spill (lk of 4000x3000: 249 against 227 us)
 
 template <int H>
-struct LkStream {
-    static constexpr int R = H + 2, SW = LKS_NT - 2 * R, WIN = 2 * H + 1;
-    static constexpr int PX = LKS_PX, NSEG = (SW + PX - 1) / PX;  // row-sum phase: PX output pixels per thread, NSEG threads per row
-    static_assert(SW > 0 && SW % 2 == 0 && PX % 2 == 0 && 2 * NSEG <= LKS_NT, "two output rows of PX-pixel segments per step");
-    static_assert(SW - 2 + WIN + PX <= LKS_NT, "the last segment's window stays inside its row of column sums");
-    static constexpr int EPAD = 2;  // float2 either side of the pair ring: the edge threads' taps stay in shared memory
-    static constexpr size_t OFF_P4 = (size_t)(6 * LKS_NT + 2 * EPAD) * 8;           // [WIN][NT] float4: products 0-3
-    static constexpr size_t OFF_P1 = OFF_P4 + (size_t)WIN * LKS_NT * 16;            // [WIN][NT] float: product 4
-    static constexpr size_t OFF_C = (OFF_P1 + (size_t)WIN * LKS_NT * 4 + 15) / 16 * 16;  // [2][5][NT] double: column sums
-    static constexpr size_t TOTAL = OFF_C + (size_t)2 * 5 * LKS_NT * 8;
+struct LkWarp {
+    static constexpr int R = H + 2, WIN = 2 * H + 1;
+    static constexpr int LANES = 30 - H;  // output lanes 1 .. LANES: the last window ends at column 61
+    static constexpr int SW = 2 * LANES;  // output columns
+    static constexpr int ROWS = 8, ST = LKW_NC + 4;  // ring rows (6 in use), floats per ring row: 2 of padding either side
+    static_assert(SW > 0 && 2 * LANES + 1 + 2 * H <= LKW_NC - 3, "windows end before the last two columns");
+    static constexpr int OFF_D = 2 * ROWS * ST;                              // floats: [WIN][3][NC] (dx, dy, dt)
+    static constexpr size_t TOTAL = (size_t)(OFF_D + WIN * 3 * LKW_NC) * 4;  // bytes
 };
+
+// Packed FP32 pairs (each half rounded as the scalar operation).
+__device__ __forceinline__ unsigned long long pk2(float2 a) { return *(unsigned long long*)&a; }
+__device__ __forceinline__ float2 upk2(unsigned long long a) { return *(float2*)&a; }
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)));
+    return upk2(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)));
+    return upk2(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
+    return upk2(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, make_float2(-1.f, -1.f), a); }
 
 // Bilinear source samples of one row (mirror addressing) and the reference texel.
 struct LkTaps {
     float s00, s10, s01, s11, a, b, r;
 };
+
+// The two window sums of a lane (2H + 1 columns from column 2l, and from
+// 2l + 1) from its own column sums c: both hold the lanes l + 1 .. l + H - 1
+// whole, summed from runs of 1, 2, 4, ... lanes.
+template <int H>
+__device__ __forceinline__ void lk_row_sums(const double (&c)[2], double (&v)[2])
+{
+    constexpr unsigned all = 0xffffffffu;
+    if constexpr (H == 0) {
+        v[0] = c[0];
+        v[1] = c[1];
+    } else {
+        const double s = c[0] + c[1];
+        double left = s, right = c[1], run = s;
+        if constexpr (H > 1) {
+            double mid = 0.0;
+            int at = 1;
+#pragma unroll
+            for (int n = 1; n <= H - 1; n *= 2) {
+                if ((H - 1) & n) {
+                    const double part = __shfl_down_sync(all, run, at);
+                    mid = at == 1 ? part : mid + part;
+                    at += n;
+                }
+                if (2 * n <= H - 1) run += __shfl_down_sync(all, run, n);
+            }
+            left += mid;
+            right += mid;
+        }
+        v[0] = left + __shfl_down_sync(all, c[0], H);
+        v[1] = right + __shfl_down_sync(all, s, H);
+    }
+}
 
 // ADJ: the adjoint-coefficient form. The same window sums at the flow
 // flow_in; instead of the update, each pixel writes lk_coeffs of the
@@ -289,195 +406,225 @@ struct LkTaps {
 // (aout, rows at a_pitch, planes a_plane bytes apart): dL/d(sxx, sxy, syy,
 // sxt, syt), zero where the forward leaves the pixel unchanged.
 template <int H, bool ADJ>
-__global__ void __launch_bounds__(LKS_NT, 512 / LKS_NT) k_lk_stream(const float2* __restrict__ flow_in, float2* __restrict__ flow_out, size_t flow_pitch,
-                                                         const float* __restrict__ src, const float* __restrict__ ref, size_t img_pitch, int W,
-                                                         int Himg, int sh, float min_det, const float2* __restrict__ gin, float* __restrict__ aout,
-                                                         size_t a_pitch, size_t a_plane)
+__global__ void __launch_bounds__(32 * LKW_WARPS, LKW_CTAS) k_lk_warp(const float2* __restrict__ flow_in, float2* __restrict__ flow_out, size_t flow_pitch,
+                                                   const float* __restrict__ src, const float* __restrict__ ref, size_t img_pitch, int W, int Himg,
+                                                   int nsx, int sh, float min_det, const float2* __restrict__ gin, float* __restrict__ aout,
+                                                   size_t a_pitch, size_t a_plane)
 {
-    using L = LkStream<H>;
-    constexpr int R = L::R, SW = L::SW, WIN = L::WIN, NT = LKS_NT, NSEG = L::NSEG, PX = L::PX;
-    extern __shared__ __align__(16) unsigned char smem[];
-    float2* E = (float2*)smem + L::EPAD;              // [6][NT] (warped source, reference), three two-row slots
-    float4* P4 = (float4*)(smem + L::OFF_P4);
-    float* P1 = (float*)(smem + L::OFF_P1);
-    double* Cs = (double*)(smem + L::OFF_C);
-    const int t = threadIdx.x;
-    const int x0 = blockIdx.x * SW, y0 = blockIdx.y * sh;
-    const int nout = min(sh, Himg - y0);
-    const int nsteps = (nout + 2 * R + 1) / 2;  // rows 0 .. 2 nsteps - 1 of the strip (one extra, mirrored, when nout is odd)
-    const int col = isa::mirror(x0 - R + t, W);
-    const float* refc = ref + col;
-    const float2* flc = flow_in + col;
+    using L = LkWarp<H>;
+    constexpr int R = L::R, WIN = L::WIN, NC = LKW_NC, ST = L::ST;
+    extern __shared__ __align__(16) float lsm_all[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int strip = blockIdx.x * LKW_WARPS + warp, sy = strip / nsx, sx = strip - sy * nsx;
+    const int x0 = sx * L::SW, y0 = sy * sh;
+    if (y0 >= Himg) return;
+    float* lsm = lsm_all + warp * (int)(L::TOTAL / 4);
+    float* Wr = lsm + 2;                    // [ROWS][ST] warped source
+    float* Rr = lsm + L::ROWS * ST + 2;     // [ROWS][ST] reference
+    float* D = lsm + L::OFF_D + 2 * lane;   // [WIN][3][NC], this lane's columns
+    const int nout = min(sh, Himg - y0), nrows = nout + 2 * R;
+    int col[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) col[k] = isa::mirror(x0 - 2 - H + lane + 32 * k, W);
     const auto erow = [&](int e) { return isa::mirror(y0 - R + e, Himg); };
-    const auto flow_at = [&](int e) { return __ldg(isa::row_ptr(flc, flow_pitch, erow(e))); };
-    const auto sample = [&](int e, float2 f, LkTaps& q) {
-        const int row = erow(e);
-        const float flx = floorf(f.x), fly = floorf(f.y);
-        const int ix = col + (int)flx, iy = row + (int)fly;
-        q.a = f.x - flx;
-        q.b = f.y - fly;
-        if ((unsigned)ix < (unsigned)(W - 1) && (unsigned)iy < (unsigned)(Himg - 1)) {
-            const float* p0 = isa::row_ptr(src, img_pitch, iy) + ix;
-            const float* p1 = isa::row_ptr(p0, img_pitch, 1);
-            q.s00 = __ldg(p0); q.s10 = __ldg(p0 + 1); q.s01 = __ldg(p1); q.s11 = __ldg(p1 + 1);
-        } else {
-            const int xa = isa::mirror(ix, W), xb = isa::mirror(ix + 1, W);
-            const float* r0 = isa::row_ptr(src, img_pitch, isa::mirror(iy, Himg));
-            const float* r1 = isa::row_ptr(src, img_pitch, isa::mirror(iy + 1, Himg));
-            q.s00 = __ldg(r0 + xa); q.s10 = __ldg(r0 + xb); q.s01 = __ldg(r1 + xa); q.s11 = __ldg(r1 + xb);
+    const auto flow_at = [&](int row, int k) { return __ldg(isa::row_ptr(flow_in, flow_pitch, row) + col[k]); };
+    // both pixels' taps: one branch for the two, so that their loads are in flight together
+    LkTaps q[2];
+    const auto sample = [&](int row, const float2 (&f)[2]) {
+        int ix[2], iy[2];
+        bool inside = true;
+        const float* rrow = isa::row_ptr(ref, img_pitch, row);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const float flx = floorf(f[k].x), fly = floorf(f[k].y);
+            ix[k] = col[k] + (int)flx;
+            iy[k] = row + (int)fly;
+            q[k].a = f[k].x - flx;
+            q[k].b = f[k].y - fly;
+            q[k].r = __ldg(rrow + col[k]);
+            inside = inside && (unsigned)ix[k] < (unsigned)(W - 1) && (unsigned)iy[k] < (unsigned)(Himg - 1);
         }
-        q.r = __ldg(isa::row_ptr(refc, img_pitch, row));
-    };
-    LkTaps qa, qb;
-    sample(0, flow_at(0), qa);
-    sample(1, flow_at(1), qb);
-    float2 fa = flow_at(2), fb = flow_at(3);
-    // the product ring starts at zero: the first 2h + 1 rows subtract nothing
-#pragma unroll 1
-    for (int k = 0; k < WIN; k++) {
-        P4[k * NT + t] = make_float4(0.f, 0.f, 0.f, 0.f);
-        P1[k * NT + t] = 0.f;
-    }
-    double cs[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    int pw = 0;                                 // product ring slot of the next product row
-    int sn = 0, s2 = 2 * NT, s1 = 4 * NT;       // pair slots: rows 2s, 2s+1 / 2s-4, 2s-3 / 2s-2, 2s-1
-    // row-sum phase: thread t < 2 NSEG sums output row (t / NSEG) of the step at columns j0 .. j0 + PX - 1
-    const int rr = t / NSEG, j0 = PX * (t - rr * NSEG);
-    const bool summer = t < 2 * NSEG;
-
-    // one product row: the centre row's pairs at c (neighbours in the ring) and above/below it in the own column
-    const auto product_row = [&](const float2* c, float2 vm2, float2 vm1, float2 vp1, float2 vp2) {
-        const float2 cm2 = c[-2], cm1 = c[-1], c0 = c[0], cp1 = c[1], cp2 = c[2];
-        // five-tap derivatives averaged over both images: ((8 (c[-1] - c[1]) + c[2] - c[-2]) / 12 of each) / 2
-        const float gx = (cp2.x - cm2.x) + (cp2.y - cm2.y) + 8.0f * ((cm1.x - cp1.x) + (cm1.y - cp1.y));
-        const float gy = (vp2.x - vm2.x) + (vp2.y - vm2.y) + 8.0f * ((vm1.x - vp1.x) + (vm1.y - vp1.y));
-        const float dx = gx * (1.0f / 24.0f), dy = gy * (1.0f / 24.0f);
-        const float dt = c0.x - c0.y;
-        const float p0 = dx * dx, p1 = dx * dy, p2 = dy * dy, p3 = dx * dt, p4 = dy * dt;
-        const float4 o4 = P4[pw * NT + t];
-        const float o1 = P1[pw * NT + t];
-        cs[0] += (double)p0 - (double)o4.x;
-        cs[1] += (double)p1 - (double)o4.y;
-        cs[2] += (double)p2 - (double)o4.z;
-        cs[3] += (double)p3 - (double)o4.w;
-        cs[4] += (double)p4 - (double)o1;
-        P4[pw * NT + t] = make_float4(p0, p1, p2, p3);
-        P1[pw * NT + t] = p4;
-        pw = pw + 1 == WIN ? 0 : pw + 1;
-    };
-    // one step: rows 2s, 2s+1 into the ring, then (DER) product rows of centres 2s-2, 2s-1, then (OUT) output rows 2s-4-2h, 2s-3-2h
-    const auto step = [&](int s, auto der, auto out) {
-        float2* en = E + sn;
-        en[t] = make_float2(isa::lerp2(qa.s00, qa.s10, qa.s01, qa.s11, qa.a, qa.b), qa.r);
-        en[NT + t] = make_float2(isa::lerp2(qb.s00, qb.s10, qb.s01, qb.s11, qb.a, qb.b), qb.r);
-        sample(2 * s + 2, fa, qa);
-        sample(2 * s + 3, fb, qb);
-        fa = flow_at(2 * s + 4);
-        fb = flow_at(2 * s + 5);
-        __syncthreads();
-        if constexpr (decltype(der)::value) {
-            const float2* e2 = E + s2 + t;  // rows 2s-4, 2s-3
-            const float2* e1 = E + s1 + t;  // rows 2s-2, 2s-1 (the centres)
-            const float2 v0 = e2[0], v1 = e2[NT], v4 = en[t], v5 = en[NT + t];
-            const float2 v2 = e1[0], v3 = e1[NT];
-            product_row(e1, v0, v1, v3, v4);
-            if constexpr (decltype(out)::value) {
+        if (inside) {
 #pragma unroll
-                for (int ch = 0; ch < 5; ch++) Cs[ch * NT + t] = cs[ch];
+            for (int k = 0; k < 2; k++) {
+                const float* p0 = isa::row_ptr(src, img_pitch, iy[k]) + ix[k];
+                const float* p1 = isa::row_ptr(p0, img_pitch, 1);
+                q[k].s00 = __ldg(p0); q[k].s10 = __ldg(p0 + 1); q[k].s01 = __ldg(p1); q[k].s11 = __ldg(p1 + 1);
             }
-            product_row(e1 + NT, v1, v2, v4, v5);
-            if constexpr (decltype(out)::value) {
+        } else {
 #pragma unroll
-                for (int ch = 0; ch < 5; ch++) Cs[(5 + ch) * NT + t] = cs[ch];
-                __syncthreads();
-                const int y = y0 + 2 * s - 4 - 2 * H + rr;  // output row
-                const int x = x0 + j0;
-                if (summer && y < y0 + nout && x < W) {
-                    const float2* irow = isa::row_ptr(ADJ ? gin : flow_in, flow_pitch, y) + x;
-                    float2 fin[PX];
+            for (int k = 0; k < 2; k++) {
+                const int xa = isa::mirror(ix[k], W), xb = isa::mirror(ix[k] + 1, W);
+                const float* r0 = isa::row_ptr(src, img_pitch, isa::mirror(iy[k], Himg));
+                const float* r1 = isa::row_ptr(src, img_pitch, isa::mirror(iy[k] + 1, Himg));
+                q[k].s00 = __ldg(r0 + xa); q[k].s10 = __ldg(r0 + xb); q[k].s01 = __ldg(r1 + xa); q[k].s11 = __ldg(r1 + xb);
+            }
+        }
+    };
+    float2 f[2];
+    {
+        const int r0 = erow(0), r1 = erow(1);
 #pragma unroll
-                    for (int k = 0; k < PX; k++) fin[k] = j0 + k < SW && x + k < W ? __ldg(irow + k) : make_float2(0.f, 0.f);
-                    // window sums of pixel j0 (2h + 1 columns from j0 + 2), then sliding by one column per pixel
-                    const double* cr = Cs + rr * 5 * NT + j0 + 2;
-                    double v[PX][5];
+        for (int k = 0; k < 2; k++) f[k] = flow_at(r0, k);
+        sample(r0, f);
 #pragma unroll
-                    for (int ch = 0; ch < 5; ch++) {
-                        const double* c = cr + ch * NT;
-                        double sum = 0.0;
+        for (int k = 0; k < 2; k++) f[k] = flow_at(r1, k);
+    }
+    // padding and the derivative ring start at zero: the first 2h + 1 rows subtract nothing
+    for (int i = lane; i < 2 * L::ROWS * ST; i += 32) lsm[i] = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < WIN * 3; i++) *(float2*)(D + i * NC) = make_float2(0.f, 0.f);
+    __syncwarp();
+    double cs[5][2];
 #pragma unroll
-                        for (int d = 0; d < WIN; d++) sum += c[d];
-                        v[0][ch] = sum;
+    for (int ch = 0; ch < 5; ch++) cs[ch][0] = cs[ch][1] = 0.0;
+    int dw = 0;  // derivative ring slot of the next centre row
+    const int xo = x0 + 2 * (lane - 1);  // first output column
+    const bool mine = lane >= 1 && lane <= L::LANES && xo < W, two = xo + 1 < W;
+    // the flow (ADJ: the upstream gradient) of the next output row
+    float2 fin[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    const auto fin_at = [&](int y) {
+        if (!mine) return;
+        const float2* p = isa::row_ptr(ADJ ? gin : flow_in, flow_pitch, y) + xo;
+        if (two && ((uintptr_t)p & 15) == 0) {
+            const float4 a = __ldg((const float4*)p);
+            fin[0] = make_float2(a.x, a.y);
+            fin[1] = make_float2(a.z, a.w);
+        } else {
+            fin[0] = __ldg(p);
+            if (two) fin[1] = __ldg(p + 1);
+        }
+    };
+
+    // row e into the ring, the next rows' loads on their way; then (OUT) the output row whose window the previous step
+    // completed, and (DER) the products of centre row e - 2 into the column sums. The row sums and the solve are one step
+    // behind the column sums: within a step they do not wait for one another.
+    const auto step = [&](int e, auto rows, auto der, auto out) {
+        constexpr bool ROW = decltype(rows)::value, DER = decltype(der)::value, OUT = decltype(out)::value;
+        if constexpr (ROW) {
+            float* w = Wr + (e & 7) * ST + lane;
+            float* r = Rr + (e & 7) * ST + lane;
 #pragma unroll
-                        for (int k = 1; k < PX; k++) v[k][ch] = sum = sum + (c[WIN + k - 1] - c[k - 1]);
-                    }
-                    const bool yin = y >= H && y < Himg - H;
-                    if constexpr (ADJ) {
-                        float* arow = isa::row_ptr(aout, a_pitch, y) + x;
+            for (int k = 0; k < 2; k++) {
+                w[32 * k] = isa::lerp2(q[k].s00, q[k].s10, q[k].s01, q[k].s11, q[k].a, q[k].b);
+                r[32 * k] = q[k].r;
+            }
+            const int r1 = erow(e + 1), r2 = erow(e + 2);
+            sample(r1, f);
 #pragma unroll
-                        for (int k = 0; k < PX; k++) {
-                            const int xk = x + k;
-                            if (j0 + k < SW && xk < W) {
-                                float co[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-                                if (yin && xk >= H && xk < W - H) lk_coeffs(fin[k], v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], min_det, co);
+            for (int k = 0; k < 2; k++) f[k] = flow_at(r2, k);
+            __syncwarp();  // row e is in; rows e - 4 .. e are read below, row e + 1 goes over row e - 7
+        }
+        double v[5][2];
+        const int y = y0 + e - 1 - 2 * R;  // output row: the previous step's centre row e - 3 is h rows below it
+        if constexpr (OUT) {
 #pragma unroll
-                                for (int ch = 0; ch < 5; ch++) ((float*)((char*)arow + ch * a_plane))[k] = co[ch];
-                            }
-                        }
-                    } else {
-                        float2* orow = isa::row_ptr(flow_out, flow_pitch, y) + x;
+            for (int ch = 0; ch < 5; ch++) lk_row_sums<H>(cs[ch], v[ch]);
+        }
+        if constexpr (DER) {
+            const float* w = Wr + 2 * lane;
+            const float* r = Rr + 2 * lane;
+            const int c = ((e - 2) & 7) * ST;
+            const auto pair = [](const float* p) { return *(const float2*)p; };
+            // centre row: columns 2l - 2 .. 2l + 3
+            const float2 wl = pair(w + c - 2), wc = pair(w + c), wh = pair(w + c + 2);
+            const float2 rl = pair(r + c - 2), rc = pair(r + c), rh = pair(r + c + 2);
+            // own columns of rows c - 2, c - 1, c + 1, c + 2
+            const int o0 = ((e - 4) & 7) * ST, o1 = ((e - 3) & 7) * ST, o2 = ((e - 1) & 7) * ST, o3 = (e & 7) * ST;
+            const float2 far = add2(sub2(pair(w + o3), pair(w + o0)), sub2(pair(r + o3), pair(r + o0)));
+            const float2 near = add2(sub2(pair(w + o1), pair(w + o2)), sub2(pair(r + o1), pair(r + o2)));
+            // five-tap derivatives averaged over both images: ((8 (c[-1] - c[1]) + c[2] - c[-2]) / 12 of each) / 2
+            const float2 c24 = make_float2(1.0f / 24.0f, 1.0f / 24.0f), c8 = make_float2(8.0f, 8.0f);
+            const float2 hfar = add2(sub2(wh, wl), sub2(rh, rl));
+            const float2 hnear = make_float2((wl.y - wc.y) + (rl.y - rc.y), (wc.x - wh.x) + (rc.x - rh.x));
+            const float2 dx = mul2(fma2(c8, hnear, hfar), c24), dy = mul2(fma2(c8, near, far), c24), dt = sub2(wc, rc);
+            float* d = D + dw * 3 * NC;
+            const float2 ex = pair(d), ey = pair(d + NC), et = pair(d + 2 * NC);
+            *(float2*)d = dx;
+            *(float2*)(d + NC) = dy;
+            *(float2*)(d + 2 * NC) = dt;
+            dw = dw + 1 == WIN ? 0 : dw + 1;
+            const auto slide = [](double (&c)[2], float2 in, float2 gone) {
+                c[0] += (double)in.x - (double)gone.x;
+                c[1] += (double)in.y - (double)gone.y;
+            };
+            slide(cs[0], mul2(dx, dx), mul2(ex, ex));
+            slide(cs[1], mul2(dx, dy), mul2(ex, ey));
+            slide(cs[2], mul2(dy, dy), mul2(ey, ey));
+            slide(cs[3], mul2(dx, dt), mul2(ex, et));
+            slide(cs[4], mul2(dy, dt), mul2(ey, et));
+        }
+        if constexpr (OUT) {
+            const bool yin = y >= H && y < Himg - H;
+            const bool on[2] = {mine && yin && xo >= H && xo < W - H, mine && yin && xo + 1 >= H && xo + 1 < W - H};
+            if constexpr (ADJ) {
+                float* arow = isa::row_ptr(aout, a_pitch, y) + xo;
 #pragma unroll
-                        for (int k = 0; k < PX; k++) {
-                            const int xk = x + k;
-                            if (j0 + k < SW && xk < W)
-                                orow[k] = yin && xk >= H && xk < W - H ? lk_update(fin[k], v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], min_det) : fin[k];
-                        }
+                for (int k = 0; k < 2; k++) {
+                    if (mine && xo + k < W) {
+                        float co[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+                        if (on[k]) lk_coeffs(fin[k], v[0][k], v[1][k], v[2][k], v[3][k], v[4][k], min_det, co);
+#pragma unroll
+                        for (int ch = 0; ch < 5; ch++) ((float*)((char*)arow + ch * a_plane))[k] = co[ch];
                     }
                 }
             } else {
-                __syncthreads();  // the next step overwrites rows 2s-4, 2s-3
+                lk_update_n<2>(fin, v, on, min_det);
+                float2* orow = isa::row_ptr(flow_out, flow_pitch, y) + xo;
+                if (mine && two && ((uintptr_t)orow & 15) == 0) {
+                    *(float4*)orow = make_float4(fin[0].x, fin[0].y, fin[1].x, fin[1].y);
+                } else if (mine) {
+                    orow[0] = fin[0];
+                    if (two) orow[1] = fin[1];
+                }
             }
+            if constexpr (ROW) fin_at(y + 1);
         }
-        const int tmp = s2;
-        s2 = s1;
-        s1 = sn;
-        sn = tmp;
     };
     using T_ = std::true_type;
     using F_ = std::false_type;
-    int s = 0;
+    int e = 0;
 #pragma unroll 1
-    for (; s < 2; s++) step(s, F_{}, F_{});
+    for (; e < 4; e++) step(e, T_{}, F_{}, F_{});
 #pragma unroll 1
-    for (; s < R; s++) step(s, T_{}, F_{});
+    for (; e <= 2 * R; e++) step(e, T_{}, T_{}, F_{});
+    fin_at(y0);
 #pragma unroll 1
-    for (; s < nsteps; s++) step(s, T_{}, T_{});
+    for (; e < nrows; e++) step(e, T_{}, T_{}, T_{});
+    step(e, F_{}, F_{}, T_{});
 }
 
-// Strip height: the grid of (column strips x row strips) CTAs should fill
-// whole waves of the CTAs resident on the device; a CTA's time grows with its
-// rows plus the 2R halo rows.
+// Strip height. A strip costs its rows plus the 2R halo rows. While an SM has
+// places left the time of a row hardly depends on how many strips it holds
+// (1.08 us for one, 1.29 us for twelve), but other streams pay for the halo's
+// extra work, so half of the cost is counted as work; beyond that strips run
+// one after the other, and their uneven ends cost about half a wave. At least
+// 8 rows: below, the halo is twice the work.
 template <int H>
 int lk_strip_rows(int W, int Himg)
 {
-    using L = LkStream<H>;
-    static int slots_by_dev[64] = {};
+    using L = LkWarp<H>;
+    static std::atomic<int> shape_by_dev[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 64;
-    int slots = slots_by_dev[dev];
-    if (slots <= 0) {
+    int shape = shape_by_dev[dev].load(std::memory_order_relaxed);
+    if (shape <= 0) {
         int nsm = 0, occ = 0;
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_lk_stream<H, false>, LKS_NT, L::TOTAL) != cudaSuccess || nsm * occ <= 0)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_lk_warp<H, false>, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL) != cudaSuccess || nsm * occ <= 0)
             return 64;
-        slots = slots_by_dev[dev] = nsm * occ;
+        shape = nsm << 8 | std::min(occ * LKW_WARPS, 255);
+        shape_by_dev[dev].store(shape, std::memory_order_relaxed);
     }
+    const long nsm = shape >> 8, occ = shape & 255;
     const long nx = (W + L::SW - 1) / L::SW;
     int best = 64;
-    long best_cost = -1;
-    for (int sh = 32; sh <= 192; sh += 2) {
+    double best_cost = -1.0;
+    for (int sh = 8; sh <= 256; sh += 2) {
         const long ny = (Himg + sh - 1) / sh;
-        const long waves = (nx * ny + slots - 1) / slots;
-        const long cost = waves * (std::min(sh, Himg) + 2 * L::R);
+        const double load = (double)((nx * ny + nsm - 1) / nsm) / (double)occ;
+        const double waves = load <= 1.0 ? 0.45 + 0.55 * load : load + 0.5;
+        const double cost = waves * (std::min(sh, Himg) + 2 * L::R);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = sh; }
     }
     return best;
@@ -487,19 +634,20 @@ template <int H>
 cudaError_t launch_lk(const float2* flow_in, float2* flow_out, size_t flow_pitch, const float* src, const float* ref, size_t img_pitch, int W, int Himg,
                       float min_det, const float2* gin, float* aout, size_t a_pitch, size_t a_plane, cudaStream_t st, int strip_rows = 0)
 {
-    using L = LkStream<H>;
+    using L = LkWarp<H>;
     const bool adj = aout != nullptr;
-    cudaError_t e = cudaFuncSetAttribute(adj ? k_lk_stream<H, true> : k_lk_stream<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)L::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(adj ? k_lk_warp<H, true> : k_lk_warp<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(LKW_WARPS * L::TOTAL));
     if (e != cudaSuccess) return e;
     const int sh = strip_rows > 0 ? strip_rows : lk_strip_rows<H>(W, Himg);
-    dim3 g((W + L::SW - 1) / L::SW, (Himg + sh - 1) / sh);
+    const int nsx = (W + L::SW - 1) / L::SW, nsy = (Himg + sh - 1) / sh;
+    const unsigned g = ((unsigned)nsx * (unsigned)nsy + LKW_WARPS - 1) / LKW_WARPS;
     if (adj)
-        k_lk_stream<H, true><<<g, LKS_NT, L::TOTAL, st>>>(flow_in, nullptr, flow_pitch, src, ref, img_pitch, W, Himg, sh, min_det, gin, aout, a_pitch,
-                                                          a_plane);
+        k_lk_warp<H, true><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, nullptr, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh, min_det,
+                                                                           gin, aout, a_pitch, a_plane);
     else
-        k_lk_stream<H, false><<<g, LKS_NT, L::TOTAL, st>>>(flow_in, flow_out, flow_pitch, src, ref, img_pitch, W, Himg, sh, min_det, nullptr, nullptr, 0,
-                                                           0);
+        k_lk_warp<H, false><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, flow_out, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh,
+                                                                            min_det, nullptr, nullptr, 0, 0);
     return cudaGetLastError();
 }
 
@@ -507,7 +655,7 @@ cudaError_t launch_lk(const float2* flow_in, float2* flow_out, size_t flow_pitch
 // f_out(p) = f_in(p) + M(p) c(p) where M, c come from the (2h+1)^2 window
 // sums of the products of dx, dy, dt at q, which are five-tap derivatives
 // (mirror addressing) of the warped source w(q) = src(q + f_in(q)) and the
-// reference. Given g = dL/df_out: k_lk_stream<h, true> writes the window
+// reference. Given g = dL/df_out: k_lk_warp<h, true> writes the window
 // sums' gradients a(p); k_box5 sums them over the window around each q
 // (A(q)); k_lk_adj_deriv turns A into gradients of dx, dy, dt at q;
 // k_lk_adj_flow applies the transposed derivative taps to get dL/dw and,

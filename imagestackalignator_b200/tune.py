@@ -1,7 +1,7 @@
 """Launch-shape autotuner for batches of uneven bursts.
 
 The shapes it chooses are the runtime knobs of isa_ctx_set_tuning: the rows
-per CTA strip of the LK iteration (flow.cu k_lk_stream) and the thread block
+per strip of the LK iteration (flow.cu k_lk_warp) and the thread block
 of the accumulation at scales other than 2 and in sample mode BILINEAR
 (merge.cu k_accumulate). Neither changes the order of any sum, so the merged
 images do not depend on them. Bursts are grouped into classes (merge scale,

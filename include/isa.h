@@ -163,7 +163,7 @@ ISA_API int isa_ctx_destroy(isa_ctx* ctx);
 ISA_API int isa_ctx_set_params(isa_ctx* ctx, const isa_params* p);
 /* Launch shapes chosen by a tuner for frames of width x height (0 x 0: any
  * size without an entry of its own); 0 in a field keeps the library's
- * choice. lk_strip_rows: rows per CTA strip of the LK iteration (else the
+ * choice. lk_strip_rows: rows per strip of the LK iteration (else the
  * wave-filling choice); acc_block_x, acc_block_y: thread block of the
  * accumulation at scales other than 1 and 2 and in sample mode BILINEAR (else
  * 32 x 8; x y <= 256). */
