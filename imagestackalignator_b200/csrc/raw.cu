@@ -13,9 +13,9 @@
 //      warp per chunk, a lane per candidate, positions only) to the first
 //      boundary at or past its end: per candidate the next chunk's
 //      candidate and the symbol count, or "stopped" at an empty table
-//      entry -- a map over PEF_K states. This stream format barely
-//      resynchronises (most of each symbol is raw difference bits), so the
-//      candidates are decoded, not guessed;
+//      entry -- a map over PEF_K states. Candidates mostly fall together
+//      within a few symbols, but none is guessed: each is followed until it
+//      has;
 //   2. the maps are chained from chunk 0's state 0 in three levels (32
 //      chunks per warp, 32 warps per block, blocks in order), then walked
 //      back down: every chunk's true start, count and local offset;
@@ -103,48 +103,126 @@ __device__ __forceinline__ void load_table(unsigned short* s, const unsigned sho
     __syncthreads();
 }
 
-// Step 1: a warp per chunk (grid-stride): the chunk's 33 words staged in
-// shared memory, lane k < PEF_K follows candidate start k (advance table only).
+// Step 1: a warp takes MAP_G chunks, their words staged in shared memory.
+// Candidates that reach the same bit stay together from there on, and most
+// do soon: with codes of 2 to 13 bits and up to 15 difference bits, 27
+// candidates are at 2.4 places on average after 128 bits and at 1.2 at the
+// chunk's end. So lane k follows candidate k of each chunk in turn over the
+// first MAP_E bits only; the places reached are listed once each, and then
+// the lanes follow the listed places of all MAP_G chunks at once to the
+// chunks' ends. Where nothing merges the list has 32 places a chunk and the
+// second part takes as long as following every candidate. Positions come
+// from the advance table only.
 constexpr int PEF_CW = 34;  // words a chunk's decode reads: 32, the next one, and one spare
+constexpr int MAP_G = 8;    // chunks a warp: 19 listed places on average, under 32 lanes
+constexpr unsigned MAP_E = 128;
 
+struct MapWarp {
+    unsigned cw[MAP_G][PEF_CW];   // words, big-endian
+    unsigned lane1[MAP_G][32];    // per candidate: place in the list, count << 8, stopped << 31
+    unsigned list[MAP_G * 32];    // place: bit | chunk << 16, then next state | count << 8
+};
+
+// Symbols from bit p to the first boundary at or past `end`; c counts them, stop: an empty table entry.
+__device__ __forceinline__ void map_walk(const unsigned* cw, const uint8_t* adv, int sh, unsigned end, unsigned& p, unsigned& c, bool& stop)
+{
+    const auto at = [&](unsigned q) {
+        const unsigned w = q >> 5;
+        return (unsigned)adv[__funnelshift_l(cw[w + 1], cw[w], q & 31) >> sh];
+    };
+    // two symbols per step while both must start before the end (a symbol is at most 32 bits)
+    while (p < end - 64) {
+        const unsigned a1 = at(p);
+        if (a1 == 0) {
+            stop = true;
+            return;
+        }
+        p += a1;
+        const unsigned a2 = at(p);
+        if (a2 == 0) {
+            c += 1;
+            stop = true;
+            return;
+        }
+        p += a2;
+        c += 2;
+    }
+    while (p < end) {
+        const unsigned a = at(p);
+        if (a == 0) {
+            stop = true;
+            return;
+        }
+        p += a;
+        c++;
+    }
+}
+
+// The maps of chunks i0 .. i0 + n - 1 (n <= MAP_G) for K candidates a chunk;
+// chunks flagged in `first` (may be null) start at bit 0 whatever the candidate.
+template <bool SWAP>
+__device__ __forceinline__ void map_chunks(MapWarp& m, const unsigned* __restrict__ words, const uint8_t* adv, int sh, const uint8_t* __restrict__ first,
+                                           int i0, int n, int K, uint8_t stop_state, uint8_t* __restrict__ nextk, uint16_t* __restrict__ cntk)
+{
+    const int k = threadIdx.x & 31;
+    for (int j = 0; j < n; j++)
+        for (int t = k; t < PEF_CW; t += 32) {
+            const unsigned w = __ldg(words + (size_t)(i0 + j) * 32 + t);
+            m.cw[j][t] = SWAP ? __byte_perm(w, 0, 0x0123) : w;
+        }
+    __syncwarp();
+    int listed = 0;
+    for (int j = 0; j < n; j++) {
+        unsigned p = first && first[i0 + j] ? 0u : (unsigned)k, c = 0;
+        bool stop = false;
+        if (k < K) map_walk(m.cw[j], adv, sh, MAP_E, p, c, stop);
+        __syncwarp();
+        // a key of its own for a lane without a place, so that all lanes take part
+        const bool live = k < K && !stop;
+        const unsigned same = __match_any_sync(0xffffffffu, live ? p : 0x10000u + k);
+        const int leader = __ffs(same) - 1;
+        const unsigned leaders = __ballot_sync(0xffffffffu, live && leader == k);
+        const unsigned place = (unsigned)(listed + __popc(leaders & ((1u << leader) - 1u)));
+        if (live && leader == k) m.list[place] = p | (unsigned)j << 16;
+        m.lane1[j][k] = (live ? place : 0u) | c << 8 | (stop ? 1u << 31 : 0u);
+        listed += __popc(leaders);
+    }
+    __syncwarp();
+    for (int q = k; q < listed; q += 32) {
+        const unsigned v = m.list[q];
+        unsigned p = v & 0xffffu, c = 0;
+        bool stop = false;
+        map_walk(m.cw[v >> 16], adv, sh, 1024, p, c, stop);
+        m.list[q] = (stop ? (unsigned)stop_state : p - 1024u) | c << 8;
+    }
+    __syncwarp();
+    if (k < K)
+        for (int j = 0; j < n; j++) {
+            const unsigned v = m.lane1[j][k], c = v >> 8 & 0x7fffffu;
+            const size_t o = (size_t)(i0 + j) * 32 + k;
+            if (v >> 31) {
+                nextk[o] = stop_state;
+                cntk[o] = (uint16_t)c;
+            } else {
+                const unsigned r = m.list[v & 255u];
+                nextk[o] = (uint8_t)(r & 255u);
+                cntk[o] = (uint16_t)(c + (r >> 8));
+            }
+        }
+    __syncwarp();
+}
+
+// Measured for 4000x3000 (24.6 MB, 188 k chunks), every candidate followed to the end -> this: 278 -> 148 us.
 __global__ void __launch_bounds__(PEF_NT) k_pef_map(const unsigned* __restrict__ words, const uint8_t* __restrict__ gadv, int nchunks,
                                                     uint8_t* __restrict__ nextk, uint16_t* __restrict__ cntk)
 {
     __shared__ __align__(16) uint8_t adv[4096];
-    __shared__ unsigned cw[PEF_NT / 32][PEF_CW];
+    __shared__ MapWarp mw[PEF_NT / 32];
     for (int i = threadIdx.x; i < 1024; i += blockDim.x) ((unsigned*)adv)[i] = ((const unsigned*)gadv)[i];
     __syncthreads();
-    const int warp = threadIdx.x >> 5, k = threadIdx.x & 31;
-    for (int i = blockIdx.x * (PEF_NT / 32) + warp; i < nchunks; i += gridDim.x * (PEF_NT / 32)) {
-        for (int t = k; t < PEF_CW; t += 32) cw[warp][t] = __ldg(words + (size_t)i * 32 + t);
-        __syncwarp();
-        if (k < PEF_K) {
-            unsigned p = (unsigned)k, c = 0;
-            bool stop = false;
-            // two symbols per step while both must start inside the chunk (a symbol is at most 27 bits)
-            while (p < PEF_CHUNK - 64) {
-                const unsigned w1 = p >> 5;
-                const unsigned a1 = adv[__funnelshift_l(cw[warp][w1 + 1], cw[warp][w1], p & 31) >> 20];
-                if (a1 == 0) { stop = true; break; }
-                p += a1;
-                const unsigned w2 = p >> 5;
-                const unsigned a2 = adv[__funnelshift_l(cw[warp][w2 + 1], cw[warp][w2], p & 31) >> 20];
-                if (a2 == 0) { c += 1; stop = true; break; }
-                p += a2;
-                c += 2;
-            }
-            while (!stop && p < PEF_CHUNK) {
-                const unsigned w = p >> 5;
-                const unsigned a = adv[__funnelshift_l(cw[warp][w + 1], cw[warp][w], p & 31) >> 20];
-                if (a == 0) { stop = true; break; }
-                p += a;
-                c++;
-            }
-            nextk[(size_t)i * 32 + k] = stop ? PEF_STOP : (uint8_t)(p - PEF_CHUNK);
-            cntk[(size_t)i * 32 + k] = (uint16_t)c;
-        }
-        __syncwarp();
-    }
+    const int warp = threadIdx.x >> 5;
+    for (int i = (blockIdx.x * (PEF_NT / 32) + warp) * MAP_G; i < nchunks; i += gridDim.x * (PEF_NT / 32) * MAP_G)
+        map_chunks<false>(mw[warp], words, adv, 20, nullptr, i, min(MAP_G, nchunks - i), PEF_K, (uint8_t)PEF_STOP, nextk, cntk);
 }
 
 // Step 2a: per block of PEF_CB = 32 x 32 chunks, the 32-chunk map of each
@@ -508,7 +586,7 @@ cudaError_t isa_launch_pef_decode(const uint8_t* data, unsigned long long nbytes
     k_pef_words<<<(unsigned)std::min<unsigned long long>((nwords + 255) / 256, 148 * 16), 256, 0, st>>>(data, nbytes, nwords, words);
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned mapg = (unsigned)std::min<long long>((nchunks + PEF_NT / 32 - 1) / (PEF_NT / 32), (long long)sms * 8);
+    const unsigned mapg = (unsigned)std::min<long long>((nchunks + PEF_NT / 32 * MAP_G - 1) / (PEF_NT / 32 * MAP_G), (long long)sms * 8);
     k_pef_map<<<mapg, PEF_NT, 0, st>>>(words, gadv, nchunks, nextk, cntk);
     k_pef_compose<<<nblocks, 1024, 0, st>>>(nextk, nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)nblocks * 32;
@@ -949,61 +1027,25 @@ __global__ void __launch_bounds__(1024) k_dngf_unstuff(const uint8_t* __restrict
     }
 }
 
-// Step 2: a warp per chunk (grid-stride), its 34 words staged big-endian in
-// shared memory; lane k follows candidate start k (0 for a part's first chunk).
+// Step 2: the maps of the chunks, as k_pef_map makes them (DF_K candidates,
+// one for a part's first chunk). 3000x2000 in 256x256 tiles, every candidate
+// followed to the end -> this: 189 -> 121 us.
 __global__ void __launch_bounds__(DF_NT) k_dngf_map(const unsigned* __restrict__ us, const uint8_t* __restrict__ gadv, int hmax, int adv_smem,
                                                     const uint8_t* __restrict__ first, int nchunks, uint8_t* __restrict__ nextk,
                                                     uint16_t* __restrict__ cntk)
 {
     extern __shared__ __align__(16) unsigned char dfm[];
-    unsigned* cwall = (unsigned*)dfm;
-    uint8_t* sadv = dfm + (DF_NT / 32) * 34 * 4;
+    MapWarp* mw = (MapWarp*)dfm;
+    uint8_t* sadv = dfm + (DF_NT / 32) * sizeof(MapWarp);
     if (adv_smem) {
         const int nw = ((1 << hmax) + 3) / 4;
         for (int i = threadIdx.x; i < nw; i += blockDim.x) ((unsigned*)sadv)[i] = ((const unsigned*)gadv)[i];
     }
     __syncthreads();
     const uint8_t* adv = adv_smem ? sadv : gadv;
-    const int warp = threadIdx.x >> 5, k = threadIdx.x & 31, sh = 32 - hmax;
-    unsigned* cw = cwall + warp * 34;
-    for (int i = blockIdx.x * (DF_NT / 32) + warp; i < nchunks; i += gridDim.x * (DF_NT / 32)) {
-        for (int t = k; t < 34; t += 32) cw[t] = bswap32(__ldg(us + (size_t)i * 32 + t));
-        __syncwarp();
-        unsigned p = first[i] ? 0u : (unsigned)k, c = 0;
-        bool stop = false;
-        // two symbols per step while both must start inside the chunk (a symbol is at most 32 bits)
-        while (p < 1024 - 64) {
-            const unsigned w1 = p >> 5;
-            const unsigned a1 = adv[__funnelshift_l(cw[w1 + 1], cw[w1], p & 31) >> sh];
-            if (a1 == 0) {
-                stop = true;
-                break;
-            }
-            p += a1;
-            const unsigned w2 = p >> 5;
-            const unsigned a2 = adv[__funnelshift_l(cw[w2 + 1], cw[w2], p & 31) >> sh];
-            if (a2 == 0) {
-                c += 1;
-                stop = true;
-                break;
-            }
-            p += a2;
-            c += 2;
-        }
-        while (!stop && p < 1024) {
-            const unsigned w = p >> 5;
-            const unsigned a = adv[__funnelshift_l(cw[w + 1], cw[w], p & 31) >> sh];
-            if (a == 0) {
-                stop = true;
-                break;
-            }
-            p += a;
-            c++;
-        }
-        nextk[(size_t)i * 32 + k] = stop ? (uint8_t)DF_STOP : (uint8_t)(p - 1024);
-        cntk[(size_t)i * 32 + k] = (uint16_t)c;
-        __syncwarp();
-    }
+    const int warp = threadIdx.x >> 5;
+    for (int i = (blockIdx.x * (DF_NT / 32) + warp) * MAP_G; i < nchunks; i += gridDim.x * (DF_NT / 32) * MAP_G)
+        map_chunks<true>(mw[warp], us, adv, 32 - hmax, first, i, min(MAP_G, nchunks - i), DF_K, (uint8_t)DF_STOP, nextk, cntk);
 }
 
 // Step 3a: per block of DF_CB = 32 x 32 chunks, the 33-state map of each warp's 32 chunks and the block's map.
@@ -1389,9 +1431,9 @@ cudaError_t isa_launch_dngf(const uint8_t* file, unsigned long long fsize, const
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int adv_smem = (1 << pl.hmax) <= 16384;
-    const size_t map_smem = (size_t)(DF_NT / 32) * 34 * 4 + (adv_smem ? pl.adv.size() : 0);
+    const size_t map_smem = (size_t)(DF_NT / 32) * sizeof(MapWarp) + (adv_smem ? pl.adv.size() : 0);
     if ((e = cudaFuncSetAttribute(k_dngf_map, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)map_smem)) != cudaSuccess) return e;
-    const unsigned mapg = (unsigned)std::min<long long>((pl.nchunks + DF_NT / 32 - 1) / (DF_NT / 32), (long long)sms * 8);
+    const unsigned mapg = (unsigned)std::min<long long>((pl.nchunks + DF_NT / 32 * MAP_G - 1) / (DF_NT / 32 * MAP_G), (long long)sms * 8);
     k_dngf_map<<<mapg, DF_NT, map_smem, st>>>((const unsigned*)us, gadv, pl.hmax, adv_smem, first, pl.nchunks, nextk, cntk);
     k_dngf_compose<<<pl.nblocks, 1024, 0, st>>>(nextk, first, pl.nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)pl.nblocks * DF_MS;
