@@ -107,15 +107,16 @@ __device__ __forceinline__ void load_table(unsigned short* s, const unsigned sho
 // Candidates that reach the same bit stay together from there on, and most
 // do soon: with codes of 2 to 13 bits and up to 15 difference bits, 27
 // candidates are at 2.4 places on average after 128 bits and at 1.2 at the
-// chunk's end. So lane k follows candidate k of each chunk in turn over the
+// chunk's end. Following 96 bits candidate by candidate is the quickest: 4000x3000
+// PEF 311 us, with 128 bits 323, with 192 bits 337. So lane k follows candidate k of each chunk in turn over the
 // first MAP_E bits only; the places reached are listed once each, and then
 // the lanes follow the listed places of all MAP_G chunks at once to the
 // chunks' ends. Where nothing merges the list has 32 places a chunk and the
 // second part takes as long as following every candidate. Positions come
 // from the advance table only.
 constexpr int PEF_CW = 34;  // words a chunk's decode reads: 32, the next one, and one spare
-constexpr int MAP_G = 8;    // chunks a warp: 19 listed places on average, under 32 lanes
-constexpr unsigned MAP_E = 128;
+constexpr int MAP_G = 8;    // chunks a warp: their listed places fill about one warp
+constexpr unsigned MAP_E = 96;
 
 struct MapWarp {
     unsigned cw[MAP_G][PEF_CW];   // words, big-endian
@@ -212,7 +213,7 @@ __device__ __forceinline__ void map_chunks(MapWarp& m, const unsigned* __restric
     __syncwarp();
 }
 
-// Measured for 4000x3000 (24.6 MB, 188 k chunks), every candidate followed to the end -> this: 278 -> 148 us.
+// Measured for 4000x3000 (24.6 MB, 188 k chunks), every candidate followed to the end -> this: 278 -> 148 us with 128 bits.
 __global__ void __launch_bounds__(PEF_NT) k_pef_map(const unsigned* __restrict__ words, const uint8_t* __restrict__ gadv, int nchunks,
                                                     uint8_t* __restrict__ nextk, uint16_t* __restrict__ cntk)
 {
@@ -1055,7 +1056,7 @@ __global__ void __launch_bounds__(1024) k_dngf_unstuff(const uint8_t* __restrict
 
 // Step 2: the maps of the chunks, as k_pef_map makes them (DF_K candidates,
 // one for a part's first chunk). 3000x2000 in 256x256 tiles, every candidate
-// followed to the end -> this: 189 -> 121 us.
+// followed to the end -> this: 189 -> 121 us with 128 bits.
 __global__ void __launch_bounds__(DF_NT) k_dngf_map(const unsigned* __restrict__ us, const uint8_t* __restrict__ gadv, int hmax, int adv_smem,
                                                     const uint8_t* __restrict__ first, int nchunks, uint8_t* __restrict__ nextk,
                                                     uint16_t* __restrict__ cntk)
