@@ -211,6 +211,33 @@ cudaError_t isa_launch_structure_tensor(const float* img, size_t pitch, int W, i
 cudaError_t isa_launch_kernel_param(const float* st3, size_t st_pitch, int W, int H, float* out, size_t out_pitch, int out_channels,
                                     float Dth, float Dtr, float kDetail, float kDenoise, float kStretch, float kShrink,
                                     cudaStream_t st);
+// The levels as the accumulation applies them: a sample enters the sums as (raw - black) scale in one multiply-add, scale
+// the power of two that brings white to 0.5 .. 1, so that the sums overflow and underflow where those of normalised samples
+// would; what is left of 1 / white, to 48 bits as the sum of two floats of one sign (the low one never zero: infinity times
+// either is infinity), is applied once per frame and channel.
+struct isa_levels {
+    float scale, nblack[3], rhigh[3], rlow[3];  // nblack: -black scale; rhigh + rlow: 1 / (white scale)
+    bool same_black;
+};
+inline isa_levels isa_make_levels(const float white[3], const float black[3])
+{
+    isa_levels l;
+    int e = 0;
+    const float wm = std::max(std::fabs(white[0]), std::max(std::fabs(white[1]), std::fabs(white[2])));
+    if (wm > 0x1p-60f && wm < 0x1p60f) std::frexp(wm, &e);
+    l.scale = std::ldexp(1.0f, -e);
+    for (int c = 0; c < 3; c++) {
+        l.nblack[c] = -black[c] * l.scale;
+        const double r = std::ldexp(1.0 / (double)white[c], e);
+        float high = (float)r;
+        if (std::fabs((double)high) > std::fabs(r)) high = std::nextafterf(high, 0.f);
+        l.rhigh[c] = high;
+        l.rlow[c] = std::isfinite(r) ? (float)(r - (double)high) : high;
+        if (l.rlow[c] == 0.f) l.rlow[c] = std::copysign(1e-45f, high);
+    }
+    l.same_black = black[0] == black[1] && black[0] == black[2];
+    return l;
+}
 // frames: host array of the frames to add, in order; frames_dev: the same list on the device (needed where nframes > 1)
 constexpr int ISA_ACC_MAX_FRAMES = 65;  // isa_ctx_create's limit
 cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const isa_frame_in* frames, const isa_frame_in* frames_dev, int nframes,

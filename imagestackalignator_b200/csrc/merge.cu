@@ -123,16 +123,29 @@ __device__ __forceinline__ int floor_div_f(int v, float s, float rs)
     return (int)(e < 0.f ? c - 1.f : c);
 }
 
+// A level per channel to one per place of the CFA (row parity * 2 + column parity).
+__device__ __forceinline__ void cfa_levels(unsigned cfa, const float (&v)[3], float (&at)[4])
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const unsigned c = (cfa >> (2 * q)) & 3;
+        at[q] = c == 0 ? v[0] : (c == 1 ? v[1] : v[2]);
+    }
+}
+
 // Any scale and CFA, tap by tap: the row and column of a tap give its sample, mask cell and CFA class (row and column
 // parity); a frame's sums are kept per class, the two classes of a row apart by predicates, and go to the channels and
-// through the black and white levels once per frame. The division by s is floor_div_f, exact where the taps' positions
-// are below 2^22 (|v| < 2^22: the frames of isa_ctx_create's limits at scale 8 stay below 2^18).
+// through the white level once per frame. Black comes off each sample, which is exact, rather than black times the weights
+// off the sums, which cancels in dark areas (largest relative error of a merge at signals of 1 to 8 over a black level of
+// 512: 8e-3 against 9e-7); SAME: one black level for all channels, a constant instead of a select per tap. The division by
+// s is floor_div_f, exact where the taps' positions are below 2^22 (|v| < 2^22: the frames of isa_ctx_create's limits at
+// scale 8 stay below 2^18).
 // Bound: instruction issue, about 1200 instructions per pixel and frame, mostly address arithmetic and predicated sums.
-// 6 x 2000x1500 at 1.5x: 1.8 ms, from 5.4 ms with per-tap divisions, indexed channels and normalisation.
-template <int KC>
+// 6 x 2000x1500 at 1.5x: 1.87 ms, from 5.4 ms with per-tap divisions, indexed channels and normalisation.
+template <int KC, bool SAME>
 __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
                                                       isa_frame_in single, size_t raw_pitch, size_t flow_pitch, size_t mask_pitch,
-                                                      const float* __restrict__ kparam, size_t kp_pitch, F3 rwhite, F3 black, float* __restrict__ acc,
+                                                      const float* __restrict__ kparam, size_t kp_pitch, isa_levels lv, float* __restrict__ acc,
                                                       float* __restrict__ wsum, size_t out_pitch, int accumulate_into)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = g.yb0 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -170,6 +183,8 @@ __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigne
         ux[d] = (isa::clampi(floor_div_f(x + d - 2 + g.ox, g.s, rs), g.cx0, g.cx1) >> 1) * 4;
         uy[d] = isa::clampi(floor_div_f(y + d - 2 + g.oy, g.s, rs), g.cy0, g.cy1) >> 1;
     }
+    float bl[4];  // black of the CFA's four places
+    cfa_levels(cfa, lv.nblack, bl);
 #pragma unroll 1
     for (int f = 0; f < nframes; f++) {
         const isa_frame_in fr = frames ? frames[f] : single;
@@ -190,6 +205,7 @@ __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigne
             const float* mr = fr.mask ? (const float*)isa::row_ptr(fr.mask, mask_pitch, uy[py]) : nullptr;
             const unsigned codes = cfa >> ((qy & 1) * 4);  // of the row's even and odd columns
             const int ce = codes & 3, co = (codes >> 2) & 3;
+            const float be = qy & 1 ? bl[2] : bl[0], bo = qy & 1 ? bl[3] : bl[1];
             float ae = 0.f, ao = 0.f, we = 0.f, wo = 0.f;
 #pragma unroll
             for (int px = 0; px < 5; px++) {
@@ -199,9 +215,10 @@ __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigne
                     cert = __ldg(mr + (ux[px] + (odd ? co : ce)));
                     if (!isfinite(cert)) cert = 0.f;
                 }
-                const float wc = __fmul_rn(wt[py * 5 + px], cert), raw = (float)__ldg(rr + qx[px]);
-                if (odd) { wo = __fadd_rn(wo, wc); ao = __fmaf_rn(wc, raw, ao); }
-                else { we = __fadd_rn(we, wc); ae = __fmaf_rn(wc, raw, ae); }
+                const float wc = __fmul_rn(wt[py * 5 + px], cert);
+                const float v = __fmaf_rn((float)__ldg(rr + qx[px]), lv.scale, SAME ? lv.nblack[0] : (odd ? bo : be));
+                if (odd) { wo = __fadd_rn(wo, wc); ao = __fmaf_rn(wc, v, ao); }
+                else { we = __fadd_rn(we, wc); ae = __fmaf_rn(wc, v, ae); }
             }
             if (qy & 1) { W[1][0] += we; W[1][1] += wo; A[1][0] += ae; A[1][1] += ao; }
             else { W[0][0] += we; W[0][1] += wo; A[0][0] += ae; A[0][1] += ao; }
@@ -212,7 +229,7 @@ __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigne
 #pragma unroll
             for (int q = 0; q < 4; q++)
                 if (((cfa >> (2 * q)) & 3) == (unsigned)c) { sa += A[q >> 1][q & 1]; sw += W[q >> 1][q & 1]; }
-            a[c] = __fmaf_rn(__fmaf_rn(-black.v[c], sw, sa), rwhite.v[c], a[c]);
+            a[c] = __fmaf_rn(sa, lv.rhigh[c], __fmaf_rn(sa, lv.rlow[c], a[c]));
             w[c] += sw;
         }
     }
@@ -744,8 +761,9 @@ cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const i
         return isa_launch_accumulate_bayer(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, white, black, acc, wsum,
                                         out_pitch, accumulate_into, st);
     if (nframes > 1 && !frames_dev) return cudaErrorInvalidValue;
-    F3 wh, rw, bl;
-    for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; rw.v[c] = (float)(1.0 / (double)white[c]); bl.v[c] = black[c]; }
+    F3 wh, bl;
+    for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; bl.v[c] = black[c]; }
+    const isa_levels lv = isa_make_levels(white, black);
     const isa_frame_in one = nframes == 1 ? frames[0] : isa_frame_in{nullptr, nullptr, nullptr};
     const isa_frame_in* list = nframes == 1 ? nullptr : frames_dev;
     if (g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
@@ -756,8 +774,9 @@ cudaError_t isa_launch_accumulate(const isa_accum_geom& g, unsigned cfa, const i
         (kparam_channels == 4 ? k_accumulate_bil<4> : k_accumulate_bil<3>)<<<grd, b, 0, st>>>(
             g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, acc, wsum, out_pitch, accumulate_into);
     else
-        (kparam_channels == 4 ? k_accumulate<4> : k_accumulate<3>)<<<grd, b, 0, st>>>(
-            g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, rw, bl, acc, wsum, out_pitch, accumulate_into);
+        (kparam_channels == 4 ? (lv.same_black ? k_accumulate<4, true> : k_accumulate<4, false>)
+                              : (lv.same_black ? k_accumulate<3, true> : k_accumulate<3, false>))<<<grd, b, 0, st>>>(
+            g, cfa, list, nframes, one, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, lv, acc, wsum, out_pitch, accumulate_into);
     return cudaGetLastError();
 }
 

@@ -30,7 +30,8 @@
 // CFA classes, which map to R, G, B through two bits per frame.
 // Per frame and channel: acc_c += (sum w cert raw - black_c sum w cert) /
 // white_c, wsum_c += sum w cert: the reference's per-tap
-// (raw - black_c) / white_c * w * cert summed over the taps of the frame.
+// (raw - black_c) / white_c * w * cert summed over the taps of the frame. (At
+// scale 1 and tap by tap black is taken off each sample.)
 // Pixels whose 3 x 3 block, mask window or flow cell reaches a border (and
 // weights so large that their sums could overflow) take a per-tap path with
 // the reference's clamps, out of line.
@@ -134,7 +135,8 @@ struct X2Args {
     size_t raw_pitch, flow_pitch, mask_pitch;
     const float4* kparam;
     size_t kp_pitch;
-    C3 rwhite, black;
+    C3 rwhite, rwlow, black;  // 1 / white: at scale 2 rwhite, rounded, at scale 1 rwhite + rwlow
+    isa_levels lv;            // of the samples tap by tap at scale 1
     float* acc;
     float* wsum;
     size_t out_pitch;
@@ -194,6 +196,7 @@ __device__ __forceinline__ float tap_weights(float k0, float k1, float k2, float
 }
 
 // One frame's sums of a pixel tap by tap at scale S (1 or 2), with the crop clamps and mirrored flow of the reference.
+// Scale 1: a is normalised; scale 2: a holds the sums of w cert raw.
 template <int S>
 __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
 {
@@ -236,11 +239,16 @@ __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
                 if (!isfinite(cert)) cert = 0.f;
             }
             const float wc = __fmul_rn(w[py + 2][d], cert);
-            const float raw = (float)__ldg(rr + qx[d]);
+            float v = (float)__ldg(rr + qx[d]);
+            if constexpr (S == 1) v = __fmaf_rn(v, A.lv.scale, c == 0 ? A.lv.nblack[0] : (c == 1 ? A.lv.nblack[1] : A.lv.nblack[2]));
 #pragma unroll
             for (int k = 0; k < 3; k++)
-                if (k == c) { s.w[k] = __fadd_rn(s.w[k], wc); s.a[k] = __fmaf_rn(wc, raw, s.a[k]); }
+                if (k == c) { s.w[k] = __fadd_rn(s.w[k], wc); s.a[k] = __fmaf_rn(wc, v, s.a[k]); }
         }
+    }
+    if constexpr (S == 1) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) s.a[c] = __fmaf_rn(s.a[c], A.lv.rhigh[c], s.a[c] * A.lv.rlow[c]);
     }
     return s;
 }
@@ -404,14 +412,16 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
 // compile-time constant; the certainty of a class is one of two values per
 // mask cell and row parity. Row patterns (YM = Y mod 2) are a template
 // parameter, uniform in a CTA; the column pattern is a select per lane.
-// Bound: instruction issue, 75 multiply-adds and about as many selects and
-// loads per pixel and frame. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
+// Black comes off each sample (see k_accumulate); SAME: one level for all
+// channels, a constant instead of four selected ones (and their spills).
+// Bound: instruction issue, 100 additions and multiply-adds and about as many
+// selects and loads per pixel and frame. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
 // with its clamps, divisions and indexed channels; one 3010x2006 frame by
 // itself 0.22 ms, from 0.72 ms. CTAs of 512 threads: 2.9 ms and 0.24 ms; at 80
 // registers (24 warps per SM) 3.0 ms.
 constexpr int X1_NT = 2 * X2_W, X1_CTAS = 4;
 
-template <int YM, bool SANE>
+template <int YM, bool SANE, bool SAME>
 __device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, const float (&w)[5][5], bool interior, float (&a)[3], float (&ws)[3])
 {
     const isa_accum_geom& g = A.g;
@@ -438,6 +448,8 @@ __device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, 
         const char* mb = mk ? mk : (const char*)g_unit_mask;
         const bool fx = k0 & 1, fy = j0 & 1;
         const bool hG = (int)(fx ^ fy) == A.bayer.g0, frr = (int)fy == A.bayer.ry;
+        const float b1 = frr ? A.black.v[0] : A.black.v[2], b2 = frr ? A.black.v[2] : A.black.v[0], bg = A.black.v[1];
+        const float bl[4] = {hG ? bg : b1, hG ? b1 : bg, hG ? b2 : bg, hG ? bg : b2};  // of the relative classes
         float Ac[4] = {0.f, 0.f, 0.f, 0.f}, Wc[4] = {0.f, 0.f, 0.f, 0.f};
         float4 M[3];
 #pragma unroll
@@ -465,7 +477,8 @@ __device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, 
             for (int d = 0; d < 5; d++) {
                 const float wc = __fmul_rn(w[r][d], k[d]);
                 const int cl = rp * 2 + (d & 1);
-                Ac[cl] = __fmaf_rn(wc, (float)__ldg(rr + d), Ac[cl]);
+                const float v = __fsub_rn((float)__ldg(rr + d), SAME ? A.black.v[0] : bl[cl]);
+                Ac[cl] = __fmaf_rn(wc, v, Ac[cl]);
                 Wc[cl] = __fadd_rn(Wc[cl], wc);
             }
         }
@@ -473,9 +486,9 @@ __device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, 
         const float NA0 = hG ? Ac[1] : Ac[0], NA1 = hG ? Ac[2] : Ac[3], NW0 = hG ? Wc[1] : Wc[0], NW1 = hG ? Wc[2] : Wc[3];
         const float ga = (hG ? Ac[0] : Ac[1]) + (hG ? Ac[3] : Ac[2]), gw = (hG ? Wc[0] : Wc[1]) + (hG ? Wc[3] : Wc[2]);
         const float ra = frr ? NA0 : NA1, ba = frr ? NA1 : NA0, rw = frr ? NW0 : NW1, bw = frr ? NW1 : NW0;
-        a[0] = __fmaf_rn(__fmaf_rn(-A.black.v[0], rw, ra), A.rwhite.v[0], a[0]);
-        a[1] = __fmaf_rn(__fmaf_rn(-A.black.v[1], gw, ga), A.rwhite.v[1], a[1]);
-        a[2] = __fmaf_rn(__fmaf_rn(-A.black.v[2], bw, ba), A.rwhite.v[2], a[2]);
+        a[0] = __fmaf_rn(ra, A.rwhite.v[0], __fmaf_rn(ra, A.rwlow.v[0], a[0]));
+        a[1] = __fmaf_rn(ga, A.rwhite.v[1], __fmaf_rn(ga, A.rwlow.v[1], a[1]));
+        a[2] = __fmaf_rn(ba, A.rwhite.v[2], __fmaf_rn(ba, A.rwlow.v[2], a[2]));
         ws[0] += rw;
         ws[1] += gw;
         ws[2] += bw;
@@ -483,7 +496,7 @@ __device__ __forceinline__ int frames_x1(const X2Args& A, int f0, int X, int Y, 
     return f;
 }
 
-template <bool SANE>
+template <bool SANE, bool SAME>
 __global__ void __launch_bounds__(X1_NT, X1_CTAS) k_accumulate_x1(const __grid_constant__ X2Args A)
 {
     const isa_accum_geom& g = A.g;
@@ -511,13 +524,13 @@ __global__ void __launch_bounds__(X1_NT, X1_CTAS) k_accumulate_x1(const __grid_c
     // the unshifted taps lie inside the crop (and with them the flow's texel in the frame), the crop holds a 5 x 5 block
     const bool interior = X - 2 >= g.cx0 && X + 2 <= g.cx1 && Y - 2 >= g.cy0 && Y + 2 <= g.cy1 && wmax < 1e30f;
     for (int f = 0;; f++) {
-        if ((Y & 1) == 0) f = frames_x1<0, SANE>(A, f, X, Y, w, interior, a, ws);  // the same for the whole CTA
-        else f = frames_x1<1, SANE>(A, f, X, Y, w, interior, a, ws);
+        if ((Y & 1) == 0) f = frames_x1<0, SANE, SAME>(A, f, X, Y, w, interior, a, ws);  // the same for the whole CTA
+        else f = frames_x1<1, SANE, SAME>(A, f, X, Y, w, interior, a, ws);
         if (f >= A.nframes) break;
         const Sums s = frame_per_tap<1>(A, f, x, y);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            a[c] += (s.a[c] - A.black.v[c] * s.w[c]) * A.rwhite.v[c];
+            a[c] += s.a[c];
             ws[c] += s.w[c];
         }
     }
@@ -567,14 +580,20 @@ cudaError_t isa_launch_accumulate_bayer(const isa_accum_geom& g, unsigned cfa, c
     for (int f = 0; f < nframes; f++) A.frames[f] = frames[f];
     A.raw_pitch = raw_pitch; A.flow_pitch = flow_pitch; A.mask_pitch = mask_pitch;
     A.kparam = (const float4*)kparam; A.kp_pitch = kparam_pitch;
-    for (int c = 0; c < 3; c++) { A.rwhite.v[c] = (float)(1.0 / (double)white[c]); A.black.v[c] = black[c]; }
+    A.lv = isa_make_levels(white, black);
+    for (int c = 0; c < 3; c++) {
+        A.rwhite.v[c] = g.s_int == 2 ? (float)(1.0 / (double)white[c]) : A.lv.rhigh[c] * A.lv.scale;
+        A.rwlow.v[c] = A.lv.rlow[c] * A.lv.scale;
+        A.black.v[c] = black[c];
+    }
     A.acc = acc; A.wsum = wsum; A.out_pitch = out_pitch; A.accumulate_into = accumulate_into;
     if (g.yb0 % 32 || g.yb0 < 0 || g.yb1 > g.Ho || g.yb1 <= g.yb0) return cudaErrorInvalidValue;
     const int rows = g.yb1 - g.yb0;  // CTA rows: four rows each in bands of 32, or two each in bands of 4
     const long long blocks = (long long)((g.Wo + X2_W - 1) / X2_W) * (g.s_int == 2 ? (rows + 31) / 32 * 8 : (rows + 3) / 4 * 2);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     const auto kernel = g.s_int == 2 ? (g.masks_finite ? k_accumulate_x2<true> : k_accumulate_x2<false>)
-                                     : (g.masks_finite ? k_accumulate_x1<true> : k_accumulate_x1<false>);
+                        : A.lv.same_black ? (g.masks_finite ? k_accumulate_x1<true, true> : k_accumulate_x1<false, true>)
+                                          : (g.masks_finite ? k_accumulate_x1<true, false> : k_accumulate_x1<false, false>);
     kernel<<<(unsigned)blocks, g.s_int == 2 ? X2_NT : X1_NT, 0, st>>>(A);
     return cudaGetLastError();
 }
