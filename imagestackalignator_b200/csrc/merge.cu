@@ -419,10 +419,11 @@ __device__ __forceinline__ void loss_sum(double lsum, double* loss)
     }
 }
 
-// Sample mode ROUND. With the black and white levels folded into the pixel's factors (v - out) h =
-// (raw - (black + white out)) (h / white) a tap costs no division; the channel's two factors come per row and column
-// parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
-// Bound: instruction issue and the mask-certainty atomics (one per tap and frame). 6 x 2000x1500 at 1.5x: 3.0 ms, from
+// Sample mode ROUND. With the white level folded into the pixel's factors, (v - out) h =
+// ((raw - black) - white out) (h / white), a tap costs no division (black comes off the sample by itself: rounded into one
+// number with white out it would cost the residual its last digits in dark areas); the channel's factors come per row and
+// column parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
+// Bound: instruction issue and the mask-certainty atomics (one per tap and frame). 6 x 2000x1500 at 1.5x: 3.1 ms, from
 // 8.0 ms with a division and branches on the channel per tap.
 template <int KC>
 __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, uns
         const float* wp = isa::row_ptr(wsum, ws_pitch, y) + 3 * x;
         const float* tp = isa::row_ptr(target, tg_pitch, y) + 3 * x;
         const float om = weight ? isa::row_ptr(weight, wt_pitch, y)[x] : 1.f;
-        float o[3], h[3];  // out in raw units (black + white out), h / white
+        float o[3], h[3];  // out in raw units over black, h / white
         bool any = false;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, uns
             lsum += (double)om * d * d;
             const float hc = wp[c] != 0.f ? 2.f * om * d / wp[c] : 0.f;
             any = any || hc != 0.f;
-            o[c] = fmaf(white.v[c], oc, black.v[c]);
+            o[c] = white.v[c] * oc;
             h[c] = hc / white.v[c];
         }
         if (x >= 1 && y >= 1 && x < g.Wo - 1 && y < g.Ho - 1 && any) {
@@ -474,6 +475,8 @@ __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, uns
                 ux[d] = (isa::clampi(floor_div_f(x + d - 2 + g.ox, g.s, rs), g.cx0, g.cx1) >> 1) * 4;
                 uy[d] = isa::clampi(floor_div_f(y + d - 2 + g.oy, g.s, rs), g.cy0, g.cy1) >> 1;
             }
+            float bl[4];  // black of the CFA's four places
+            cfa_levels(cfa, black.v, bl);
 #pragma unroll 1
             for (int f = 0; f < nframes; f++) {
                 const isa_frame_in fr = frames[f];
@@ -495,12 +498,13 @@ __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, uns
                     const int ce = codes & 3, co = (codes >> 2) & 3;
                     const float oe = ce == 0 ? o[0] : (ce == 1 ? o[1] : o[2]), he = ce == 0 ? h[0] : (ce == 1 ? h[1] : h[2]);
                     const float oo = co == 0 ? o[0] : (co == 1 ? o[1] : o[2]), ho = co == 0 ? h[0] : (co == 1 ? h[1] : h[2]);
+                    const float be = qy & 1 ? bl[2] : bl[0], bo = qy & 1 ? bl[3] : bl[1];
                     const size_t mrow = (size_t)uy[py] * mask_pitch;
 #pragma unroll
                     for (int px = 0; px < 5; px++) {
                         const int t = py * 5 + px;
                         const bool odd = qx[px] & 1;
-                        const float r = ((float)__ldg(rr + qx[px]) - (odd ? oo : oe)) * (odd ? ho : he);
+                        const float r = (((float)__ldg(rr + qx[px]) - (odd ? bo : be)) - (odd ? oo : oe)) * (odd ? ho : he);
                         float cert = 1.f;
                         if (fr.mask) {
                             const size_t at = mrow + 4u * (unsigned)(ux[px] + (odd ? co : ce));

@@ -1,4 +1,4 @@
-"""Black and white levels in the accumulation.
+"""Black and white levels in the accumulation and its gradient.
 
 Black comes off every sample before any rounding, so a constant added to the
 samples and to black changes nothing, bit for bit, however dark the frame;
@@ -9,7 +9,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from imagestackalignator_b200 import isa
+from imagestackalignator_b200 import isa, params as P
 from test_gpu_accumulate_forms import CASES
 
 pytestmark = pytest.mark.gpu
@@ -109,3 +109,41 @@ def test_large_weights_stay_finite(cuda, scale, kc):
     assert np.isfinite(a).all() and np.isfinite(w).all() and w.max() > 1e35
     a, w = a[1:-1, 1:-1].astype(np.float64), w[1:-1, 1:-1].astype(np.float64)
     assert (w > 0).all() and (a / w).max() <= 1.0 + 1e-5 and (a / w).min() >= -512.0 / 15871.0 - 1e-5
+
+
+@pytest.mark.parametrize("scale", [1.5, 3.0])
+def test_gradient_keeps_the_last_digits_of_dark_frames(cuda, scale):
+    """Equal frames of 1 .. 20 over black: no motion, full certainty, so raising the samples and black by 49152 changes
+    nothing the gradient depends on. The two gradients differ by the order of the FP32 atomic sums alone: a term per
+    weighted pixel and tap, 200 in all, so 200 * 2^-24 = 1.2e-5 of the terms' magnitudes; a few pixels are weighted, so that
+    rounding errors do not average out."""
+    import torch
+    W, H, n = 336, 336, 3
+    rng = np.random.default_rng(4)
+    img = (10.0 + 6.0 * np.sin(np.arange(W)[None, :] / 9.0) * np.cos(np.arange(H)[:, None] / 7.0) + rng.uniform(-3, 3, (H, W))).round()
+    frame = np.clip(img, 1, 20).astype(np.uint16)
+    p = P.MergeParams(merge_scale=scale)
+    outs, grads, losses = [], [], []
+    for lift in (0, 49152):
+        info = isa.IsaRawInfo()
+        info.width, info.height = W, H
+        info.cfa[:] = (0, 1, 1, 2)
+        info.black[:] = (float(lift),) * 3
+        info.white[:] = (15871.0,) * 3
+        info.camera_white[:] = (1.0,) * 3
+        info.noise_alpha, info.noise_beta = 1e-3, 8e-6
+        raw = torch.from_numpy(np.repeat((frame + np.uint16(lift))[None], n, 0).view(np.int16)).cuda()
+        m = isa.Merger(W, H, n, p)
+        out = m.merge(raw, info).clone()
+        if not outs:
+            target = (out * 0.5).contiguous()
+            om = torch.zeros(out.shape[:2], device="cuda")
+            om[150:152, 200:204] = 1.0
+        _, loss, grad = m.backward(raw, info, target, weight=om)
+        outs.append(out.cpu().numpy())
+        grads.append(grad[:6])
+        losses.append(loss)
+        m.close()
+    assert np.array_equal(outs[0], outs[1]) and losses[0] == losses[1]
+    assert np.abs(grads[0]).max() > 0
+    assert np.allclose(grads[0], grads[1], rtol=1e-4, atol=1.2e-5 * np.abs(grads[0]).max()), (grads[0], grads[1])
