@@ -9,10 +9,11 @@
 // the integer pixel and the sub-pixel flow part so that FP32 keeps full
 // sub-pixel precision far from the origin.
 //
-// k_lk_warp fuses one reference iteration (warp, Set(0) x3, derivatives,
-// lucasKanadeOptim) for a vertical strip of the image, walking down it row by
-// row: FP32 gradient products, FP64 sliding window sums, and the 2x2
-// pseudo-inverse in FP64.
+// k_lk_warp and k_lk_stream fuse one reference iteration (warp, Set(0) x3,
+// derivatives, lucasKanadeOptim) for a vertical strip of the image, walking
+// down it row by row: FP32 gradient products, FP64 sliding window sums, and
+// the 2x2 pseudo-inverse in FP64; by warps for windows of 3 to 19 columns, by
+// CTAs for the others.
 #include "isa_internal.cuh"
 
 #include <algorithm>
@@ -107,16 +108,21 @@ __device__ __forceinline__ bool lk_matrix(double a, double b, double d, double m
     return r.ok;
 }
 
-// Out of line: the per-pixel kernel calls it only where lk_update_n's quick
-// decisions are not certain.
-__device__ __noinline__ float2 lk_update(float2 f, double a, double b, double d, double sxt, double syt, double min_det)
+__device__ __forceinline__ float2 lk_solve(float2 f, double a, double b, double d, double sxt, double syt, double min_det)
 {
     double m0, m1, m2, m3;
     if (!lk_matrix(a, b, d, min_det, m0, m1, m2, m3)) return f;
     return lk_apply(f, m0, m1, m2, m3, sxt, syt);
 }
 
-// lk_update at the pixels of f (v: the five window sums of each; on: pixels to
+// Out of line: k_lk_warp calls it only where lk_update_n's quick decisions
+// are not certain.
+__device__ __noinline__ float2 lk_update(float2 f, double a, double b, double d, double sxt, double syt, double min_det)
+{
+    return lk_solve(f, a, b, d, sxt, syt, min_det);
+}
+
+// lk_solve at the pixels of f (v: the five window sums of each; on: pixels to
 // update). The usual case, a well-conditioned matrix, runs without a branch at
 // all pixels side by side: a branch or a division's own slow path between
 // them would put their FP64 chains one after the other. The largest
@@ -161,7 +167,7 @@ __device__ __forceinline__ void lk_update_n(float2 (&f)[N], const double (&v)[5]
         if (on[k]) f[k] = g[k];
 }
 
-// Adjoint of lk_update at one pixel for the upstream gradient g of the
+// Adjoint of lk_solve at one pixel for the upstream gradient g of the
 // updated flow: with delta = M c (c = (sxt, syt)) and gamma = M^T g, the
 // window sums get dL/dsxx = -gamma_x delta_x, dL/dsxy = -(gamma_x delta_y +
 // gamma_y delta_x), dL/dsyy = -gamma_y delta_y, dL/dsxt = gamma_x,
@@ -289,7 +295,7 @@ __global__ void k_lk_sums(float2* flow, size_t flow_pitch, const float* __restri
         }
     }
     float2* fp = isa::row_ptr(flow, flow_pitch, y) + x;
-    *fp = lk_update(*fp, sxx, sxy, syy, sxt, syt, min_det);
+    *fp = lk_solve(*fp, sxx, sxy, syy, sxt, syt, min_det);
 }
 
 // Streaming form of one reference iteration (warp, Set(0) x3, derivatives,
@@ -594,37 +600,257 @@ __global__ void __launch_bounds__(32 * LKW_WARPS, LKW_CTAS) k_lk_warp(const floa
     step(e, F_{}, F_{}, T_{});
 }
 
-// Strip height. A strip costs its rows plus the 2R halo rows. While an SM has
-// places left the time of a row hardly depends on how many strips it holds
-// (1.08 us for one, 1.29 us for twelve), but other streams pay for the halo's
-// extra work, so half of the cost is counted as work; beyond that strips run
-// one after the other, and their uneven ends cost about half a wave. At least
-// 8 rows: below, the halo is twice the work.
+// The same iteration by a CTA of LKS_NT threads for a strip of LKS_NT columns
+// (SW = LKS_NT - 2R of output, R = h + 2), thread t at image column x0 - R + t
+// (mirrored at the border), two rows per step: the warped source and the
+// reference of the two rows go into a ring of six rows of pairs in shared
+// memory; after a barrier, derivatives at the two centre rows, FP32 products
+// and vertical window sums as above (the products themselves in the ring);
+// after a second barrier, row window sums of 2h + 1 column sums read from
+// shared memory, two pixels a thread, and the solve. The sums hold the same
+// products, so both kernels round to the same flow.
+//
+// It takes windows of 21 columns and more, where the warp's 64 columns leave
+// 40 to 30 of output (this strip's 128: 104 to 94) and 8 warps fit an SM, and
+// window 1, whose matrices are all singular, so that every pixel takes the
+// out-of-line solve, which the warp's 12 places an SM hide less well than the
+// 16 here. One iteration, warp -> this: window 21 1024x768 54 -> 50 us,
+// 4000x3000 428 -> 365, 6016x4000 643 -> 640; window 31 1024x768 80 -> 58,
+// 4000x3000 520 -> 570; window 1 2000x1500 125 -> 103, 4000x3000 474 -> 326.
+// Windows 3 to 19 are faster by warps: window 19 4000x3000 287 against 346.
+constexpr int LKS_NT = 128, LKS_PX = 2;
+
+template <int H>
+struct LkStream {
+    static constexpr int R = H + 2, SW = LKS_NT - 2 * R, WIN = 2 * H + 1;
+    static constexpr int PX = LKS_PX, NSEG = (SW + PX - 1) / PX;  // row-sum phase: PX output pixels per thread, NSEG threads per row
+    static_assert(SW > 0 && SW % 2 == 0 && PX % 2 == 0 && 2 * NSEG <= LKS_NT, "two output rows of PX-pixel segments per step");
+    static_assert(SW - 2 + WIN + PX <= LKS_NT, "the last segment's window stays inside its row of column sums");
+    static constexpr int EPAD = 2;  // float2 either side of the pair ring: the edge threads' taps stay in shared memory
+    static constexpr size_t OFF_P4 = (size_t)(6 * LKS_NT + 2 * EPAD) * 8;           // [WIN][NT] float4: products 0-3
+    static constexpr size_t OFF_P1 = OFF_P4 + (size_t)WIN * LKS_NT * 16;            // [WIN][NT] float: product 4
+    static constexpr size_t OFF_C = (OFF_P1 + (size_t)WIN * LKS_NT * 4 + 15) / 16 * 16;  // [2][5][NT] double: column sums
+    static constexpr size_t TOTAL = OFF_C + (size_t)2 * 5 * LKS_NT * 8;
+};
+
+template <int H, bool ADJ>
+__global__ void __launch_bounds__(LKS_NT, 512 / LKS_NT) k_lk_stream(const float2* __restrict__ flow_in, float2* __restrict__ flow_out, size_t flow_pitch,
+                                                         const float* __restrict__ src, const float* __restrict__ ref, size_t img_pitch, int W,
+                                                         int Himg, int sh, float min_det, const float2* __restrict__ gin, float* __restrict__ aout,
+                                                         size_t a_pitch, size_t a_plane)
+{
+    using L = LkStream<H>;
+    constexpr int R = L::R, SW = L::SW, WIN = L::WIN, NT = LKS_NT, NSEG = L::NSEG, PX = L::PX;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float2* E = (float2*)smem + L::EPAD;              // [6][NT] (warped source, reference), three two-row slots
+    float4* P4 = (float4*)(smem + L::OFF_P4);
+    float* P1 = (float*)(smem + L::OFF_P1);
+    double* Cs = (double*)(smem + L::OFF_C);
+    const int t = threadIdx.x;
+    const int x0 = blockIdx.x * SW, y0 = blockIdx.y * sh;
+    const int nout = min(sh, Himg - y0);
+    const int nsteps = (nout + 2 * R + 1) / 2;  // rows 0 .. 2 nsteps - 1 of the strip (one extra, mirrored, when nout is odd)
+    const int col = isa::mirror(x0 - R + t, W);
+    const float* refc = ref + col;
+    const float2* flc = flow_in + col;
+    const auto erow = [&](int e) { return isa::mirror(y0 - R + e, Himg); };
+    const auto flow_at = [&](int e) { return __ldg(isa::row_ptr(flc, flow_pitch, erow(e))); };
+    const auto sample = [&](int e, float2 f, LkTaps& q) {
+        const int row = erow(e);
+        const float flx = floorf(f.x), fly = floorf(f.y);
+        const int ix = col + (int)flx, iy = row + (int)fly;
+        q.a = f.x - flx;
+        q.b = f.y - fly;
+        if ((unsigned)ix < (unsigned)(W - 1) && (unsigned)iy < (unsigned)(Himg - 1)) {
+            const float* p0 = isa::row_ptr(src, img_pitch, iy) + ix;
+            const float* p1 = isa::row_ptr(p0, img_pitch, 1);
+            q.s00 = __ldg(p0); q.s10 = __ldg(p0 + 1); q.s01 = __ldg(p1); q.s11 = __ldg(p1 + 1);
+        } else {
+            const int xa = isa::mirror(ix, W), xb = isa::mirror(ix + 1, W);
+            const float* r0 = isa::row_ptr(src, img_pitch, isa::mirror(iy, Himg));
+            const float* r1 = isa::row_ptr(src, img_pitch, isa::mirror(iy + 1, Himg));
+            q.s00 = __ldg(r0 + xa); q.s10 = __ldg(r0 + xb); q.s01 = __ldg(r1 + xa); q.s11 = __ldg(r1 + xb);
+        }
+        q.r = __ldg(isa::row_ptr(refc, img_pitch, row));
+    };
+    LkTaps qa, qb;
+    sample(0, flow_at(0), qa);
+    sample(1, flow_at(1), qb);
+    float2 fa = flow_at(2), fb = flow_at(3);
+    // the product ring starts at zero: the first 2h + 1 rows subtract nothing
+#pragma unroll 1
+    for (int k = 0; k < WIN; k++) {
+        P4[k * NT + t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        P1[k * NT + t] = 0.f;
+    }
+    double cs[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    int pw = 0;                                 // product ring slot of the next product row
+    int sn = 0, s2 = 2 * NT, s1 = 4 * NT;       // pair slots: rows 2s, 2s+1 / 2s-4, 2s-3 / 2s-2, 2s-1
+    // row-sum phase: thread t < 2 NSEG sums output row (t / NSEG) of the step at columns j0 .. j0 + PX - 1
+    const int rr = t / NSEG, j0 = PX * (t - rr * NSEG);
+    const bool summer = t < 2 * NSEG;
+
+    // one product row: the centre row's pairs at c (neighbours in the ring) and above/below it in the own column
+    const auto product_row = [&](const float2* c, float2 vm2, float2 vm1, float2 vp1, float2 vp2) {
+        const float2 cm2 = c[-2], cm1 = c[-1], c0 = c[0], cp1 = c[1], cp2 = c[2];
+        // five-tap derivatives averaged over both images: ((8 (c[-1] - c[1]) + c[2] - c[-2]) / 12 of each) / 2
+        const float gx = (cp2.x - cm2.x) + (cp2.y - cm2.y) + 8.0f * ((cm1.x - cp1.x) + (cm1.y - cp1.y));
+        const float gy = (vp2.x - vm2.x) + (vp2.y - vm2.y) + 8.0f * ((vm1.x - vp1.x) + (vm1.y - vp1.y));
+        const float dx = gx * (1.0f / 24.0f), dy = gy * (1.0f / 24.0f);
+        const float dt = c0.x - c0.y;
+        const float p0 = dx * dx, p1 = dx * dy, p2 = dy * dy, p3 = dx * dt, p4 = dy * dt;
+        const float4 o4 = P4[pw * NT + t];
+        const float o1 = P1[pw * NT + t];
+        cs[0] += (double)p0 - (double)o4.x;
+        cs[1] += (double)p1 - (double)o4.y;
+        cs[2] += (double)p2 - (double)o4.z;
+        cs[3] += (double)p3 - (double)o4.w;
+        cs[4] += (double)p4 - (double)o1;
+        P4[pw * NT + t] = make_float4(p0, p1, p2, p3);
+        P1[pw * NT + t] = p4;
+        pw = pw + 1 == WIN ? 0 : pw + 1;
+    };
+    // one step: rows 2s, 2s+1 into the ring, then (DER) product rows of centres 2s-2, 2s-1, then (OUT) output rows 2s-4-2h, 2s-3-2h
+    const auto step = [&](int s, auto der, auto out) {
+        float2* en = E + sn;
+        en[t] = make_float2(isa::lerp2(qa.s00, qa.s10, qa.s01, qa.s11, qa.a, qa.b), qa.r);
+        en[NT + t] = make_float2(isa::lerp2(qb.s00, qb.s10, qb.s01, qb.s11, qb.a, qb.b), qb.r);
+        sample(2 * s + 2, fa, qa);
+        sample(2 * s + 3, fb, qb);
+        fa = flow_at(2 * s + 4);
+        fb = flow_at(2 * s + 5);
+        __syncthreads();
+        if constexpr (decltype(der)::value) {
+            const float2* e2 = E + s2 + t;  // rows 2s-4, 2s-3
+            const float2* e1 = E + s1 + t;  // rows 2s-2, 2s-1 (the centres)
+            const float2 v0 = e2[0], v1 = e2[NT], v4 = en[t], v5 = en[NT + t];
+            const float2 v2 = e1[0], v3 = e1[NT];
+            product_row(e1, v0, v1, v3, v4);
+            if constexpr (decltype(out)::value) {
+#pragma unroll
+                for (int ch = 0; ch < 5; ch++) Cs[ch * NT + t] = cs[ch];
+            }
+            product_row(e1 + NT, v1, v2, v4, v5);
+            if constexpr (decltype(out)::value) {
+#pragma unroll
+                for (int ch = 0; ch < 5; ch++) Cs[(5 + ch) * NT + t] = cs[ch];
+                __syncthreads();
+                const int y = y0 + 2 * s - 4 - 2 * H + rr;  // output row
+                const int x = x0 + j0;
+                if (summer && y < y0 + nout && x < W) {
+                    const float2* irow = isa::row_ptr(ADJ ? gin : flow_in, flow_pitch, y) + x;
+                    float2 fin[PX];
+#pragma unroll
+                    for (int k = 0; k < PX; k++) fin[k] = j0 + k < SW && x + k < W ? __ldg(irow + k) : make_float2(0.f, 0.f);
+                    // window sums of pixel j0 (2h + 1 columns from j0 + 2), then sliding by one column per pixel
+                    const double* cr = Cs + rr * 5 * NT + j0 + 2;
+                    double v[PX][5];
+#pragma unroll
+                    for (int ch = 0; ch < 5; ch++) {
+                        const double* c = cr + ch * NT;
+                        double sum = 0.0;
+#pragma unroll
+                        for (int d = 0; d < WIN; d++) sum += c[d];
+                        v[0][ch] = sum;
+#pragma unroll
+                        for (int k = 1; k < PX; k++) v[k][ch] = sum = sum + (c[WIN + k - 1] - c[k - 1]);
+                    }
+                    const bool yin = y >= H && y < Himg - H;
+                    if constexpr (ADJ) {
+                        float* arow = isa::row_ptr(aout, a_pitch, y) + x;
+#pragma unroll
+                        for (int k = 0; k < PX; k++) {
+                            const int xk = x + k;
+                            if (j0 + k < SW && xk < W) {
+                                float co[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+                                if (yin && xk >= H && xk < W - H) lk_coeffs(fin[k], v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], min_det, co);
+#pragma unroll
+                                for (int ch = 0; ch < 5; ch++) ((float*)((char*)arow + ch * a_plane))[k] = co[ch];
+                            }
+                        }
+                    } else {
+                        float2* orow = isa::row_ptr(flow_out, flow_pitch, y) + x;
+#pragma unroll
+                        for (int k = 0; k < PX; k++) {
+                            const int xk = x + k;
+                            if (j0 + k < SW && xk < W)
+                                orow[k] = yin && xk >= H && xk < W - H ? lk_solve(fin[k], v[k][0], v[k][1], v[k][2], v[k][3], v[k][4], min_det) : fin[k];
+                        }
+                    }
+                }
+            } else {
+                __syncthreads();  // the next step overwrites rows 2s-4, 2s-3
+            }
+        }
+        const int tmp = s2;
+        s2 = s1;
+        s1 = sn;
+        sn = tmp;
+    };
+    using T_ = std::true_type;
+    using F_ = std::false_type;
+    int s = 0;
+#pragma unroll 1
+    for (; s < 2; s++) step(s, F_{}, F_{});
+#pragma unroll 1
+    for (; s < R; s++) step(s, T_{}, F_{});
+#pragma unroll 1
+    for (; s < nsteps; s++) step(s, T_{}, T_{});
+}
+
+// Which kernel a window takes (above).
+template <int H>
+constexpr bool lk_by_warps = H >= 1 && H <= 9;
+
+// Strip height of the CTA strips: the grid of (column strips x row strips)
+// CTAs should fill whole waves of the CTAs resident on the device; a CTA's
+// time grows with its rows plus the 2R halo rows.
+//
+// Strip height of the warps. A strip costs its rows plus the 2R halo rows.
+// While an SM has places left the time of a row hardly depends on how many
+// strips it holds (1.08 us for one, 1.29 us for twelve), but other streams pay
+// for the halo's extra work, so half of the cost is counted as work (less from
+// window 17 on, whose halo is longer: 1024x768 at window 19 55 -> 46 us with
+// 12 rows instead of 22); beyond that strips run one after the other, and their
+// uneven ends cost about half a wave. At least 8 rows: below, the halo is twice
+// the work. In a window of 3 columns many pixels take the out-of-line solve,
+// and unevenly: several short strips a place, not one long one (2000x1500
+// 60 -> 57 us, 4000x3000 181 -> 164).
 template <int H>
 int lk_strip_rows(int W, int Himg)
 {
-    using L = LkWarp<H>;
     static std::atomic<int> shape_by_dev[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 64;
     int shape = shape_by_dev[dev].load(std::memory_order_relaxed);
     if (shape <= 0) {
         int nsm = 0, occ = 0;
-        if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_lk_warp<H, false>, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL) != cudaSuccess || nsm * occ <= 0)
-            return 64;
-        shape = nsm << 8 | std::min(occ * LKW_WARPS, 255);
+        cudaError_t e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) {
+            if constexpr (lk_by_warps<H>)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_lk_warp<H, false>, 32 * LKW_WARPS, LKW_WARPS * LkWarp<H>::TOTAL);
+            else
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_lk_stream<H, false>, LKS_NT, LkStream<H>::TOTAL);
+        }
+        if (e != cudaSuccess || nsm * occ <= 0) return 64;
+        shape = nsm << 8 | std::min(lk_by_warps<H> ? occ * LKW_WARPS : occ, 255);
         shape_by_dev[dev].store(shape, std::memory_order_relaxed);
     }
     const long nsm = shape >> 8, occ = shape & 255;
-    const long nx = (W + L::SW - 1) / L::SW;
     int best = 64;
     double best_cost = -1.0;
-    for (int sh = 8; sh <= 256; sh += 2) {
+    for (int sh = lk_by_warps<H> ? 8 : 32; sh <= (lk_by_warps<H> ? 256 : 192); sh += 2) {
         const long ny = (Himg + sh - 1) / sh;
-        const double load = (double)((nx * ny + nsm - 1) / nsm) / (double)occ;
-        const double waves = load <= 1.0 ? 0.45 + 0.55 * load : load + 0.5;
-        const double cost = waves * (std::min(sh, Himg) + 2 * L::R);
+        double waves;
+        if constexpr (lk_by_warps<H>) {
+            const long nx = (W + LkWarp<H>::SW - 1) / LkWarp<H>::SW;
+            const double load = (double)((nx * ny + nsm - 1) / nsm) / (double)occ, work = H <= 7 ? 0.55 : 0.4;
+            waves = H == 1 ? load + 0.6 : (load <= 1.0 ? 1.0 - work + work * load : load + 0.5);
+        } else {
+            const long nx = (W + LkStream<H>::SW - 1) / LkStream<H>::SW;
+            waves = (double)((nx * ny + nsm * occ - 1) / (nsm * occ));
+        }
+        const double cost = waves * (std::min(sh, Himg) + 2 * (H + 2));
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = sh; }
     }
     return best;
@@ -634,20 +860,34 @@ template <int H>
 cudaError_t launch_lk(const float2* flow_in, float2* flow_out, size_t flow_pitch, const float* src, const float* ref, size_t img_pitch, int W, int Himg,
                       float min_det, const float2* gin, float* aout, size_t a_pitch, size_t a_plane, cudaStream_t st, int strip_rows = 0)
 {
-    using L = LkWarp<H>;
     const bool adj = aout != nullptr;
-    cudaError_t e = cudaFuncSetAttribute(adj ? k_lk_warp<H, true> : k_lk_warp<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(LKW_WARPS * L::TOTAL));
-    if (e != cudaSuccess) return e;
     const int sh = strip_rows > 0 ? strip_rows : lk_strip_rows<H>(W, Himg);
-    const int nsx = (W + L::SW - 1) / L::SW, nsy = (Himg + sh - 1) / sh;
-    const unsigned g = ((unsigned)nsx * (unsigned)nsy + LKW_WARPS - 1) / LKW_WARPS;
-    if (adj)
-        k_lk_warp<H, true><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, nullptr, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh, min_det,
-                                                                           gin, aout, a_pitch, a_plane);
-    else
-        k_lk_warp<H, false><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, flow_out, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh,
-                                                                            min_det, nullptr, nullptr, 0, 0);
+    if constexpr (lk_by_warps<H>) {
+        using L = LkWarp<H>;
+        cudaError_t e = cudaFuncSetAttribute(adj ? k_lk_warp<H, true> : k_lk_warp<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(LKW_WARPS * L::TOTAL));
+        if (e != cudaSuccess) return e;
+        const int nsx = (W + L::SW - 1) / L::SW, nsy = (Himg + sh - 1) / sh;
+        const unsigned g = ((unsigned)nsx * (unsigned)nsy + LKW_WARPS - 1) / LKW_WARPS;
+        if (adj)
+            k_lk_warp<H, true><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, nullptr, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh,
+                                                                               min_det, gin, aout, a_pitch, a_plane);
+        else
+            k_lk_warp<H, false><<<g, 32 * LKW_WARPS, LKW_WARPS * L::TOTAL, st>>>(flow_in, flow_out, flow_pitch, src, ref, img_pitch, W, Himg, nsx, sh,
+                                                                                min_det, nullptr, nullptr, 0, 0);
+    } else {
+        using L = LkStream<H>;
+        cudaError_t e = cudaFuncSetAttribute(adj ? k_lk_stream<H, true> : k_lk_stream<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)L::TOTAL);
+        if (e != cudaSuccess) return e;
+        const dim3 g((W + L::SW - 1) / L::SW, (Himg + sh - 1) / sh);
+        if (adj)
+            k_lk_stream<H, true><<<g, LKS_NT, L::TOTAL, st>>>(flow_in, nullptr, flow_pitch, src, ref, img_pitch, W, Himg, sh, min_det, gin, aout, a_pitch,
+                                                              a_plane);
+        else
+            k_lk_stream<H, false><<<g, LKS_NT, L::TOTAL, st>>>(flow_in, flow_out, flow_pitch, src, ref, img_pitch, W, Himg, sh, min_det, nullptr, nullptr,
+                                                               0, 0);
+    }
     return cudaGetLastError();
 }
 
