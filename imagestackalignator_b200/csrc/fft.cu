@@ -455,7 +455,7 @@ cudaError_t isa_launch_fft_rows_r2c(const float* in, size_t in_pitch, float2* sp
     const size_t smem = (size_t)(2 * padded(W / 2) + max_prime(pn)) * sizeof(float2);  // two padded buffers of W / 2, prime roots
     if (smem > 227 * 1024 || (W & 1) || pn.n != W / 2 || ((uintptr_t)in & 7) || (in_pitch & 7) || ((uintptr_t)spec & 7) || (spec_pitch & 7))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_fft_rows_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = isa_allow_smem(k_fft_rows_r2c, smem);
     if (e != cudaSuccess) return e;
     k_fft_rows_r2c<<<H, kRowThreads, smem, st>>>(in, in_pitch, spec, spec_pitch, W, pn, tw_n, tw_w);
     return cudaGetLastError();
@@ -467,7 +467,7 @@ cudaError_t isa_launch_fft_rows_c2r(const float2* spec, size_t spec_pitch, float
     const size_t smem = (size_t)(2 * padded(W / 2) + max_prime(pn)) * sizeof(float2);  // N + 1 bins / scratch, conj Z', prime roots
     if (smem > 227 * 1024 || (W & 1) || pn.n != W / 2 || ((uintptr_t)out & 7) || (out_pitch & 7) || ((uintptr_t)spec & 7) || (spec_pitch & 7))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_fft_rows_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = isa_allow_smem(k_fft_rows_c2r, smem);
     if (e != cudaSuccess) return e;
     k_fft_rows_c2r<<<H, kRowThreads, smem, st>>>(spec, spec_pitch, out, out_pitch, W, pn, tw_n, tw_w, clamp01, kfrom, kscale);
     return cudaGetLastError();
@@ -486,7 +486,7 @@ cudaError_t isa_launch_fft_cols(float2* spec, size_t spec_pitch, int W, int H, i
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     C = std::max(1, std::min(C, (ncols + nsm - 1) / nsm));
     const size_t smem = ((size_t)2 * C * padded(H) + max_prime(ph)) * sizeof(float2);
-    cudaError_t e = cudaFuncSetAttribute(k_fft_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = isa_allow_smem(k_fft_cols, smem);
     if (e != cudaSuccess) return e;
     if (ncols < 0 || ncols > W / 2 + 1) return cudaErrorInvalidValue;
     if (ncols == 0) return cudaSuccess;

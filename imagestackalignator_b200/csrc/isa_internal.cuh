@@ -10,6 +10,17 @@
 
 #define ISA_DEV __device__ __forceinline__
 
+// Leave to launch `kernel` (no static shared memory) with `smem` bytes of dynamic shared memory. The attribute is a
+// property of the kernel that all host threads share, so where sizes depend on the input it is always set to the most a
+// block can have: set to the size at hand, one thread could lower it between another's call here and its launch.
+constexpr size_t ISA_SMEM_MAX = 227 * 1024;
+template <class K>
+inline cudaError_t isa_allow_smem(K* kernel, size_t smem)
+{
+    if (smem > ISA_SMEM_MAX) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ISA_SMEM_MAX);
+}
+
 namespace isa {
 
 // ---- pitched access ------------------------------------------------------

@@ -617,7 +617,7 @@ cudaError_t isa_launch_pef_decode(const uint8_t* data, unsigned long long nbytes
     k_pef_map<<<mapg, PEF_NT, 0, st>>>(words, gadv, nchunks, nextk, cntk);
     k_pef_compose<<<nblocks, 1024, 0, st>>>(nextk, nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)nblocks * 32;
-    cudaError_t e = cudaFuncSetAttribute(k_pef_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(chain_smem, 1));
+    cudaError_t e = isa_allow_smem(k_pef_chain, chain_smem);
     if (e != cudaSuccess) return e;
     k_pef_chain<<<1, 256, chain_smem, st>>>(block_map, nblocks, block_in, final_state);
     k_pef_walk<<<nblocks, 1024, 0, st>>>(nextk, cntk, sub_map, block_in, nchunks, start, loc, block_total);
@@ -930,7 +930,7 @@ cudaError_t isa_launch_dng(const uint8_t* file, unsigned long long fsize, int co
         // the tables go to shared memory too when they fit beside the warps' buffers
         const int ntab = ((size_t)ntables * 2 + 16 + per_warp <= 200 * 1024) ? ntables : 0;
         const size_t smem = (size_t)(ntab * 2 + 15) / 16 * 16 + per_warp;
-        cudaError_t e = cudaFuncSetAttribute(k_dng_lj92, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = isa_allow_smem(k_dng_lj92, smem);
         if (e != cudaSuccess) return e;
         k_dng_lj92<<<(nparts + DNG_WARPS - 1) / DNG_WARPS, 32 * DNG_WARPS, smem, st>>>(A, jwide_max, ntab);
     } else {
@@ -1462,19 +1462,19 @@ cudaError_t isa_launch_dngf(const uint8_t* file, unsigned long long fsize, const
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int adv_smem = (1 << pl.hmax) <= 16384;
     const size_t map_smem = (size_t)(DF_NT / 32) * sizeof(MapWarp) + (adv_smem ? pl.adv.size() : 0);
-    if ((e = cudaFuncSetAttribute(k_dngf_map, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)map_smem)) != cudaSuccess) return e;
+    if ((e = isa_allow_smem(k_dngf_map, map_smem)) != cudaSuccess) return e;
     const unsigned mapg = (unsigned)std::min<long long>((pl.nchunks + DF_NT / 32 * MAP_G - 1) / (DF_NT / 32 * MAP_G), (long long)sms * 8);
     k_dngf_map<<<mapg, DF_NT, map_smem, st>>>((const unsigned*)us, gadv, pl.hmax, adv_smem, first, pl.nchunks, nextk, cntk);
     k_dngf_compose<<<pl.nblocks, 1024, 0, st>>>(nextk, first, pl.nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)pl.nblocks * DF_MS;
-    if ((e = cudaFuncSetAttribute(k_dngf_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem)) != cudaSuccess) return e;
+    if ((e = isa_allow_smem(k_dngf_chain, chain_smem)) != cudaSuccess) return e;
     k_dngf_chain<<<1, 256, chain_smem, st>>>(block_map, pl.nblocks, block_in);
     k_dngf_walk<<<pl.nblocks, 1024, 0, st>>>(nextk, cntk, sub_map, block_in, first, pl.nchunks, sin, loc, block_total);
     k_pef_scan<<<1, 1024, 0, st>>>(block_total, pl.nblocks, boff);
     k_dngf_parts<<<(nparts + 255) / 256, 256, 0, st>>>(d_parts, nparts, pl.nchunks, pl.nblocks, nextk, sin, loc, boff, g0, d_anomaly);
     const int tab_smem = (1 << pl.hmax) <= 8192;
     const size_t emit_smem = (size_t)(DF_NT * 33 + 4) * 4 + (tab_smem ? ((size_t)1 + ((size_t)1 << pl.hmax)) * 2 : 0);
-    if ((e = cudaFuncSetAttribute(k_dngf_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem)) != cudaSuccess) return e;
+    if ((e = isa_allow_smem(k_dngf_emit, emit_smem)) != cudaSuccess) return e;
     k_dngf_emit<<<(pl.nchunks + DF_NT - 1) / DF_NT, DF_NT, emit_smem, st>>>((const unsigned*)us, (unsigned long long)pl.nchunks * 32 + 64, d_parts, d_cs,
                                                                           nparts, pl.nchunks, pl.nblocks, sin, loc, boff, g0, gtab, pl.hmax, tab_smem,
                                                                           large, diff);

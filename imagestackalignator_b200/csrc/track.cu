@@ -840,7 +840,7 @@ cudaError_t isa_launch_solve(const int* row_a, const int* row_b, const int* row_
     if (per_warp > 227 * 1024) return cudaErrorInvalidValue;
     const int wpc = (int)std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / per_warp));
     const size_t smem = per_warp * wpc;
-    cudaError_t e = cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = isa_allow_smem(k_solve, smem);
     if (e != cudaSuccess) return e;
     const int ntiles = tcx * tcy;
     k_solve<<<(ntiles + wpc - 1) / wpc, 32 * wpc, smem, st>>>(row_a, row_b, row_sign, N0, m, n1, grids, grid_pitch, grid_stride, row_grid, tcx, tcy,
