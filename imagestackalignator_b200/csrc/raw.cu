@@ -103,20 +103,26 @@ __device__ __forceinline__ void load_table(unsigned short* s, const unsigned sho
     __syncthreads();
 }
 
-// Step 1: a warp takes MAP_G chunks, their words staged in shared memory.
+// Step 1: a warp takes up to MAP_G chunks, their words staged in shared memory.
 // Candidates that reach the same bit stay together from there on, and most
 // do soon: with codes of 2 to 13 bits and up to 15 difference bits, 27
 // candidates are at 2.4 places on average after 128 bits and at 1.2 at the
-// chunk's end. Following 96 bits candidate by candidate is the quickest: 4000x3000
-// PEF 311 us, with 128 bits 323, with 192 bits 337. So lane k follows candidate k of each chunk in turn over the
-// first MAP_E bits only; the places reached are listed once each, and then
-// the lanes follow the listed places of all MAP_G chunks at once to the
+// chunk's end. So lane k follows candidate k of each chunk in turn over the
+// first MAP_E bits only (96 are the quickest: 4000x3000 PEF 311 us, with 128
+// bits 323, with 192 bits 337); the places reached are listed once each, and
+// then the lanes follow the listed places of all its chunks at once to the
 // chunks' ends. Where nothing merges the list has 32 places a chunk and the
 // second part takes as long as following every candidate. Positions come
 // from the advance table only.
 constexpr int PEF_CW = 34;  // words a chunk's decode reads: 32, the next one, and one spare
 constexpr int MAP_G = 8;    // chunks a warp: their listed places fill about one warp
 constexpr unsigned MAP_E = 96;
+
+// Chunks a warp takes of nchunks: fewer than MAP_G where that would leave an SM under 24 warps, since the first part is a
+// chain over a warp's chunks. Whole decodes, eight chunks a warp -> by this rule: PEF 336x336 (1.7 k chunks) 121 -> 109 us,
+// 800x640 (7.9 k) 133 -> 121; DNG 800x640 391 -> 348, 1000x700 (11 k) 377 -> 352; at 30 k chunks eight a warp are as quick
+// as four, from 46 k on quicker (PEF 2400x1700: 172 against 185 with four, 226 with one).
+int map_group(long long nchunks, int sms) { return (int)std::max<long long>(1, std::min<long long>(MAP_G, nchunks / ((long long)sms * 24))); }
 
 struct MapWarp {
     unsigned cw[MAP_G][PEF_CW];   // words, big-endian
@@ -215,15 +221,35 @@ __device__ __forceinline__ void map_chunks(MapWarp& m, const unsigned* __restric
 
 // Measured for 4000x3000 (24.6 MB, 188 k chunks), every candidate followed to the end -> this: 278 -> 148 us with 128 bits.
 __global__ void __launch_bounds__(PEF_NT) k_pef_map(const unsigned* __restrict__ words, const uint8_t* __restrict__ gadv, int nchunks,
-                                                    uint8_t* __restrict__ nextk, uint16_t* __restrict__ cntk)
+                                                    int group, uint8_t* __restrict__ nextk, uint16_t* __restrict__ cntk)
 {
     __shared__ __align__(16) uint8_t adv[4096];
     __shared__ MapWarp mw[PEF_NT / 32];
     for (int i = threadIdx.x; i < 1024; i += blockDim.x) ((unsigned*)adv)[i] = ((const unsigned*)gadv)[i];
     __syncthreads();
     const int warp = threadIdx.x >> 5;
-    for (int i = (blockIdx.x * (PEF_NT / 32) + warp) * MAP_G; i < nchunks; i += gridDim.x * (PEF_NT / 32) * MAP_G)
-        map_chunks<false>(mw[warp], words, adv, 20, nullptr, i, min(MAP_G, nchunks - i), PEF_K, (uint8_t)PEF_STOP, nextk, cntk);
+    for (int i = (blockIdx.x * (PEF_NT / 32) + warp) * group; i < nchunks; i += gridDim.x * (PEF_NT / 32) * group)
+        map_chunks<false>(mw[warp], words, adv, 20, nullptr, i, min(group, nchunks - i), PEF_K, (uint8_t)PEF_STOP, nextk, cntk);
+}
+
+// The maps of chunks c0 .. c0 + n - 1 (n <= 1024; 32 bytes a chunk) to put(chunk, byte, four states), by 1024 threads, a
+// thread's eight loads side by side (32 loads of a byte, which the compiler may leave one after the other, make the two
+// composing kernels 10 to 20 us; this, 6 and 7).
+template <class F>
+__device__ __forceinline__ void compose_load(const uint8_t* __restrict__ nextk, int c0, int n, F&& put)
+{
+    const unsigned* src = (const unsigned*)(nextk + (size_t)c0 * 32);
+    unsigned v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int t = threadIdx.x + k * 1024;
+        v[k] = t < n * 8 ? src[t] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int t = threadIdx.x + k * 1024;
+        if (t < n * 8) put(t >> 3, (t & 7) * 4, v[k]);
+    }
 }
 
 // Step 2a: per block of PEF_CB = 32 x 32 chunks, the 32-chunk map of each
@@ -231,10 +257,10 @@ __global__ void __launch_bounds__(PEF_NT) k_pef_map(const unsigned* __restrict__
 __global__ void __launch_bounds__(1024) k_pef_compose(const uint8_t* __restrict__ nextk, int nchunks, uint8_t* __restrict__ sub_map,
                                                       uint8_t* __restrict__ block_map)
 {
-    __shared__ uint8_t m[PEF_CB][32];
+    __shared__ __align__(4) uint8_t m[PEF_CB][32];
     __shared__ uint8_t sm[32][32];
     const int c0 = blockIdx.x * PEF_CB, n = min(PEF_CB, nchunks - c0);
-    for (int t = threadIdx.x; t < n * 32; t += blockDim.x) m[t >> 5][t & 31] = nextk[(size_t)c0 * 32 + t];
+    compose_load(nextk, c0, n, [&](int q, int b, unsigned v) { *(unsigned*)&m[q][b] = v; });
     __syncthreads();
     const int warp = threadIdx.x >> 5, j = threadIdx.x & 31;
     unsigned s = j < PEF_K ? (unsigned)j : PEF_STOP;
@@ -362,23 +388,32 @@ __global__ void __launch_bounds__(1024) k_pef_scan(const unsigned* __restrict__ 
 // runs of their own, so every 2-byte store of a warp was 32 sectors; whole
 // groups of four leave as one 8-byte store, what stands before the first
 // group and after the last one value by value (the whole decode of a
-// 4000x3000 PEF frame 395 -> 332 us, of a 3000x2000 DNG 547 -> 535 us).
+// 4000x3000 PEF frame 395 -> 332 us, of a 3000x2000 DNG 547 -> 535 us). A
+// value costs 32-bit arithmetic and one branch: with 64-bit indexes and the
+// first group told apart at every value, DNG 1000x700 took 360 us against 352
+// (2-byte stores 351), 4000x2000 550 against 538.
 struct RunOut {
-    uint16_t* base;               // 8-byte aligned
-    unsigned long long g, first;  // next index, the first whole group's
-    unsigned long long acc;       // the last four values
-    __device__ RunOut(uint16_t* b, unsigned long long at) : base(b), g(at), first((at + 3) & ~3ull), acc(0) {}
+    uint16_t* group;         // the current group of four (8-byte aligned)
+    unsigned g, skip;        // next index (from the first group's start); places of the current group before the run
+    unsigned long long acc;  // the last four values
+    __device__ RunOut(uint16_t* base, unsigned long long at) : group(base + (at & ~3ull)), g((unsigned)at & 3), skip((unsigned)at & 3), acc(0) {}
+    // index of the n-th value from here on (a chunk has at most 1024)
+    __device__ __forceinline__ unsigned after(unsigned long long n) const { return g + (unsigned)(n < 0x7fffffffull ? n : 0x7fffffffull); }
     __device__ __forceinline__ void put(int d)
     {
         acc = acc >> 16 | (unsigned long long)(uint16_t)d << 48;
-        if (g < first) base[g] = (uint16_t)d;
-        else if ((g & 3) == 3) *(unsigned long long*)(base + g - 3) = acc;
-        g++;
+        if ((g++ & 3) == 3) {
+            if (skip == 0) *(unsigned long long*)group = acc;
+            else
+                for (; skip < 4; skip++) group[skip] = (uint16_t)(acc >> 16 * skip);
+            skip = 0;
+            group += 4;
+        }
     }
     __device__ __forceinline__ void end() const
     {
-        const int n = g > first ? (int)(g & 3) : 0;
-        for (int i = 0; i < n; i++) base[g - n + i] = (uint16_t)(acc >> 16 * (4 - n + i));
+        const unsigned n = g & 3;
+        for (unsigned i = skip; i < n; i++) group[i] = (uint16_t)(acc >> 16 * (4 - n + i));
     }
 };
 
@@ -406,7 +441,8 @@ __global__ void __launch_bounds__(PEF_NT) k_pef_emit(const unsigned* __restrict_
     unsigned p = (unsigned)(start[i] - (unsigned long long)i * PEF_CHUNK);
     const unsigned* cb = cw + 33 * t;
     RunOut run((uint16_t*)diff, o);
-    while (p < PEF_CHUNK && run.g < limit) {
+    const unsigned end = run.after(limit - o);
+    while (p < PEF_CHUNK && run.g < end) {
         const unsigned w = p >> 5;
         const unsigned x = __funnelshift_l(cb[w + 1 + ((w + 1) >> 5)], cb[w], p & 31);
         int a;
@@ -613,8 +649,9 @@ cudaError_t isa_launch_pef_decode(const uint8_t* data, unsigned long long nbytes
     k_pef_words<<<(unsigned)std::min<unsigned long long>((nwords + 255) / 256, 148 * 16), 256, 0, st>>>(data, nbytes, nwords, words);
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned mapg = (unsigned)std::min<long long>((nchunks + PEF_NT / 32 * MAP_G - 1) / (PEF_NT / 32 * MAP_G), (long long)sms * 8);
-    k_pef_map<<<mapg, PEF_NT, 0, st>>>(words, gadv, nchunks, nextk, cntk);
+    const int group = map_group(nchunks, sms);
+    const unsigned mapg = (unsigned)std::min<long long>((nchunks + PEF_NT / 32 * group - 1) / (PEF_NT / 32 * group), (long long)sms * 8);
+    k_pef_map<<<mapg, PEF_NT, 0, st>>>(words, gadv, nchunks, group, nextk, cntk);
     k_pef_compose<<<nblocks, 1024, 0, st>>>(nextk, nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)nblocks * 32;
     cudaError_t e = isa_allow_smem(k_pef_chain, chain_smem);
@@ -1058,7 +1095,7 @@ __global__ void __launch_bounds__(1024) k_dngf_unstuff(const uint8_t* __restrict
 // one for a part's first chunk). 3000x2000 in 256x256 tiles, every candidate
 // followed to the end -> this: 189 -> 121 us with 128 bits.
 __global__ void __launch_bounds__(DF_NT) k_dngf_map(const unsigned* __restrict__ us, const uint8_t* __restrict__ gadv, int hmax, int adv_smem,
-                                                    const uint8_t* __restrict__ first, int nchunks, uint8_t* __restrict__ nextk,
+                                                    const uint8_t* __restrict__ first, int nchunks, int group, uint8_t* __restrict__ nextk,
                                                     uint16_t* __restrict__ cntk)
 {
     extern __shared__ __align__(16) unsigned char dfm[];
@@ -1071,8 +1108,8 @@ __global__ void __launch_bounds__(DF_NT) k_dngf_map(const unsigned* __restrict__
     __syncthreads();
     const uint8_t* adv = adv_smem ? sadv : gadv;
     const int warp = threadIdx.x >> 5;
-    for (int i = (blockIdx.x * (DF_NT / 32) + warp) * MAP_G; i < nchunks; i += gridDim.x * (DF_NT / 32) * MAP_G)
-        map_chunks<true>(mw[warp], us, adv, 32 - hmax, first, i, min(MAP_G, nchunks - i), DF_K, (uint8_t)DF_STOP, nextk, cntk);
+    for (int i = (blockIdx.x * (DF_NT / 32) + warp) * group; i < nchunks; i += gridDim.x * (DF_NT / 32) * group)
+        map_chunks<true>(mw[warp], us, adv, 32 - hmax, first, i, min(group, nchunks - i), DF_K, (uint8_t)DF_STOP, nextk, cntk);
 }
 
 // Step 3a: per block of DF_CB = 32 x 32 chunks, the 33-state map of each warp's 32 chunks and the block's map.
@@ -1082,7 +1119,10 @@ __global__ void __launch_bounds__(1024) k_dngf_compose(const uint8_t* __restrict
     __shared__ uint8_t m[DF_CB][33];
     __shared__ uint8_t sm[32][DF_MS];
     const int c0 = blockIdx.x * DF_CB, n = min(DF_CB, nchunks - c0);
-    for (int t = threadIdx.x; t < n * 32; t += blockDim.x) m[t >> 5][t & 31] = nextk[(size_t)c0 * 32 + t];
+    compose_load(nextk, c0, n, [&](int q, int b, unsigned v) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) m[q][b + k] = (uint8_t)(v >> 8 * k);
+    });
     __syncthreads();
     for (int q = threadIdx.x; q < n; q += blockDim.x) m[q][32] = first[c0 + q] ? m[q][0] : (uint8_t)DF_STOP;
     __syncthreads();
@@ -1236,8 +1276,8 @@ __global__ void __launch_bounds__(DF_NT) k_dngf_emit(const unsigned* __restrict_
     const unsigned* cb = cw + 33 * threadIdx.x;
     const int sh = 32 - hmax;
     RunOut run(diff, P.sbase + o);
-    const unsigned long long send = P.sbase + S;
-    while (p < 1024 && run.g < send) {
+    const unsigned end = run.after(S - o);
+    while (p < 1024 && run.g < end) {
         const unsigned w = p >> 5;
         const unsigned x = __funnelshift_l(cb[w + 1 + ((w + 1) >> 5)], cb[w], p & 31);
         const unsigned e = tab[x >> sh];
@@ -1463,8 +1503,9 @@ cudaError_t isa_launch_dngf(const uint8_t* file, unsigned long long fsize, const
     const int adv_smem = (1 << pl.hmax) <= 16384;
     const size_t map_smem = (size_t)(DF_NT / 32) * sizeof(MapWarp) + (adv_smem ? pl.adv.size() : 0);
     if ((e = isa_allow_smem(k_dngf_map, map_smem)) != cudaSuccess) return e;
-    const unsigned mapg = (unsigned)std::min<long long>((pl.nchunks + DF_NT / 32 * MAP_G - 1) / (DF_NT / 32 * MAP_G), (long long)sms * 8);
-    k_dngf_map<<<mapg, DF_NT, map_smem, st>>>((const unsigned*)us, gadv, pl.hmax, adv_smem, first, pl.nchunks, nextk, cntk);
+    const int group = map_group(pl.nchunks, sms);
+    const unsigned mapg = (unsigned)std::min<long long>((pl.nchunks + DF_NT / 32 * group - 1) / (DF_NT / 32 * group), (long long)sms * 8);
+    k_dngf_map<<<mapg, DF_NT, map_smem, st>>>((const unsigned*)us, gadv, pl.hmax, adv_smem, first, pl.nchunks, group, nextk, cntk);
     k_dngf_compose<<<pl.nblocks, 1024, 0, st>>>(nextk, first, pl.nchunks, sub_map, block_map);
     const size_t chain_smem = (size_t)pl.nblocks * DF_MS;
     if ((e = isa_allow_smem(k_dngf_chain, chain_smem)) != cudaSuccess) return e;
