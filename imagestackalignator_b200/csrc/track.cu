@@ -13,6 +13,7 @@
 #include "isa_internal.cuh"
 #include <float.h>
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 namespace {
@@ -306,8 +307,8 @@ cudaError_t launch_track_ts(const float* const* frames, size_t pitch, int Wl, in
 // registers, so the chain pair table -> pre-shift -> frame table -> tile loads
 // is off the critical path.
 // Bound: the FMA pipe (2 lane operations per template pixel and shift), busy
-// about 60 %; 12 warps per SM (15 KB of shared memory each) leave the chains of
-// staging and minimum search partly exposed. All 190 pairs of 20 x 6016x4000:
+// about 60 %; 12 warps per SM (S = 2, 15 KB of shared memory each; at S = 5 and 6,
+// 19 and 21 KB, 8) leave the chains of staging and minimum search partly exposed. All 190 pairs of 20 x 6016x4000:
 // tile alignment (four levels and solves) 29.1 -> 23.0 ms.
 template <int T, int S>
 struct WarpDims {
@@ -549,9 +550,20 @@ cudaError_t launch_track_warp(const float* const* frames, size_t pitch, int Wl, 
     cudaError_t e = cudaFuncSetAttribute(k_track_warp<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
     if (e != cudaSuccess) return e;
     // pairs per warp: up to 16 (the start of a run is not overlapped), fewer while the runs would not fill the device's
-    // 148 x 12 resident warps eight times over; the runs of a tile about equally long
+    // places (148 x 12 warps at S = 2) eight times over; the runs of a tile about equally long
+    static std::atomic<int> places_by_dev[64];
+    int dev = 0, places = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) places = places_by_dev[dev].load(std::memory_order_relaxed);
+    if (places <= 0) {
+        int nsm = 0, occ = 0;
+        if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_track_warp<T, S>, 32 * L::WARPS, L::BYTES)) != cudaSuccess) return e;
+        places = std::max(1, nsm * occ * L::WARPS);
+        if (dev >= 0 && dev < 64) places_by_dev[dev].store(places, std::memory_order_relaxed);
+    }
     const long long items = (long long)npairs * tcx * tcy;
-    const int most = (int)std::max<long long>(1, std::min<long long>({16, npairs, items / (148 * 12 * 8)}));
+    const int most = (int)std::max<long long>(1, std::min<long long>({16, npairs, items / ((long long)places * 8)}));
     const int nruns = (npairs + most - 1) / most, run = (npairs + nruns - 1) / nruns;
     const long long warps = (long long)nruns * tcx * tcy, blocks = (warps + L::WARPS - 1) / L::WARPS;
     if (warps > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -782,12 +794,18 @@ __global__ void k_optimal(const float2* __restrict__ x, int n1, int tcx, int tcy
 
 }  // namespace
 
-// A warp per (pair, tile) or a CTA: the same sums, so the choice is one of time. Few items leave the device idle with a
-// warp each (300 items of 32 x 32, S = 2: 6.8 us against 5.5 us with a CTA each; 2660: 15.3 against 14.3), many keep it
-// busier (7448: 31.1 against 31.3; 19964: 71 against 74; 82908: 252 against 294; S = 4: 27.0 against 26.7 at 2660, 589
-// against 664 at 82908). For 16 x 16 tiles the warp's fixed work weighs more (S = 2, 31668 items: 57 against 60 us;
-// 11310: 25.8 against 24.5), and at S = 4, where its lane groups share nine shift rows unevenly, 205128 items take 625
-// against 643 us but 82908 take 273 against 262. Other tile sizes: a CTA each.
+// A warp per (pair, tile) or a CTA: the same sums, so the choice is one of time. Few items (pairs x tiles) leave the device
+// idle with a warp each, many keep it busier. Us by CTAs / by warps, at the numbers of items where the line is drawn:
+//   T 32, S 1: 44415  101 /  99, 69564  158 / 160, 82908  185 / 162  (below, up to a quarter slower: 23188  58 / 73)
+//         S 2:  7130   29 /  29,  8883   35 /  34, 82908  287 / 242
+//         S 3: never: 23188  128 / 146, 82908  441 / 484, 322896  1701 / 1725 (its 7 shift rows take three passes of 3)
+//         S 4:  2961   29 /  29,  7130   62 /  58, 82908  660 / 576
+//         S 5:  8883  101 / 101, 11532  130 / 129, 82908  897 / 850
+//         S 6: 44415  644 / 660, 69192 1000 / 981, 82908 1197 / 1182
+//   T 16, S 1: never: 44415  40 /  62, 322896  267 / 318
+//         S 2: 34596   62 /  66, 44415   77 /  76, 82908  140 / 126
+//         S 4 (nine shift rows over two lane groups): 82908  259 / 259, 322896  996 / 946
+// Other tile sizes: a CTA each.
 #define ISA_TRACK_CASE(TT, SS, FROM)                                                                                                            \
     if (T == TT && S == SS) {                                                                                                                     \
         if constexpr ((FROM) > 0)                                                                                                                 \
@@ -804,9 +822,9 @@ cudaError_t isa_launch_track(const float* const* frames, size_t img_pitch, int W
 {
     if (npairs <= 0 || tcx <= 0 || tcy <= 0) return cudaSuccess;
     const long long items = (long long)npairs * tcx * tcy;
-    ISA_TRACK_CASE(32, 1, 6000) ISA_TRACK_CASE(32, 2, 6000) ISA_TRACK_CASE(32, 3, 6000) ISA_TRACK_CASE(32, 4, 3000)
-    ISA_TRACK_CASE(32, 5, 3000) ISA_TRACK_CASE(32, 6, 3000)
-    ISA_TRACK_CASE(16, 1, 24000) ISA_TRACK_CASE(16, 2, 24000) ISA_TRACK_CASE(16, 4, 0) ISA_TRACK_CASE(16, 8, 0)
+    ISA_TRACK_CASE(32, 1, 80000) ISA_TRACK_CASE(32, 2, 8000) ISA_TRACK_CASE(32, 3, 0) ISA_TRACK_CASE(32, 4, 3000)
+    ISA_TRACK_CASE(32, 5, 12000) ISA_TRACK_CASE(32, 6, 70000)
+    ISA_TRACK_CASE(16, 1, 0) ISA_TRACK_CASE(16, 2, 50000) ISA_TRACK_CASE(16, 4, 0) ISA_TRACK_CASE(16, 8, 0)
     ISA_TRACK_CASE(64, 2, 0)
     ISA_TRACK_CASE(8, 2, 0) ISA_TRACK_CASE(8, 4, 0)
     return cudaErrorInvalidValue;
