@@ -1,16 +1,18 @@
 """Launch-shape autotuner for batches of uneven bursts.
 
 The shapes it chooses are the runtime knobs of isa_ctx_set_tuning: the rows
-per strip of the LK iteration (flow.cu k_lk_warp) and the thread block
-of the accumulation at scales other than 2 and in sample mode BILINEAR
-(merge.cu k_accumulate). Neither changes the order of any sum, so the merged
-images do not depend on them. Bursts are grouped into classes (merge scale,
+per strip of the LK iteration (flow.cu k_lk_warp, k_lk_stream) and the thread
+block of the accumulation where a general kernel runs (merge.cu k_accumulate,
+k_accumulate_bil: scales other than 1 and 2, sample mode BILINEAR, CFAs other
+than Bayer's). Neither changes the order of any sum, so the merged images do
+not depend on them. Bursts are grouped into classes (merge scale,
 aspect ratio, frame area rounded to 2 MP); for one burst of each class every
 candidate is timed on the device (CUDA events, after a warm-up merge) by
-coordinate search (strip rows first, then the block); a shape replaces the
-library's own choice only when it is at least 3 % faster, and the winner
-applies to every frame size of the class. Results are cached as JSON keyed by class
-and device name, so a later run on the same kind of GPU reuses them.
+coordinate search (strip rows first, then the block, where a kernel reads it);
+a shape replaces the library's own choice only when it is at least 3 % faster,
+and the winner applies to every frame size of the class. Results are cached as
+JSON keyed by device name, the kernels they were timed on, class and what else
+the shapes depend on, so a later run on the same kind of GPU reuses them.
 """
 from __future__ import annotations
 
@@ -18,7 +20,8 @@ import json
 import os
 from typing import Dict, List, Optional
 
-LK_ROWS = (0, 32, 48, 64, 96, 128)
+KERNELS = "lk-warp-1"  # changes with the kernels that read the shapes: a shape timed on another one says nothing
+LK_ROWS = (0, 8, 16, 24, 32, 48, 64, 96, 128)
 ACC_BLOCKS = ((0, 0), (32, 4), (64, 4), (16, 16), (128, 2))
 MARGIN = 0.03  # a shape replaces the library's choice only when at least this much faster
 
@@ -30,6 +33,16 @@ def default_cache_path() -> str:
 def burst_class(width: int, height: int, scale: float) -> str:
     aspect = "3:2" if abs(width / height - 1.5) < abs(width / height - 4 / 3) else "4:3"
     return f"s{scale:g}-{aspect}-{int(round(width * height / 2e6)) * 2}MP"
+
+
+def reads_block(params, cfa) -> bool:
+    """Whether the accumulation of such a merge reads the thread block: not the kernels of Bayer frames at scales 1 and 2."""
+    if params.sample_mode != 0:
+        return True
+    scale = float(params.merge_scale) or (2.0 if params.super_resolution else 1.0)
+    c = tuple(cfa)
+    bayer = c in ((0, 1, 1, 2), (2, 1, 1, 0), (1, 0, 2, 1), (1, 2, 0, 1))
+    return not (bayer and scale in (1.0, 2.0))
 
 
 def _device_name() -> str:
@@ -84,12 +97,16 @@ def tune(merger, items: List[dict], cache_path: Optional[str] = None, reps: int 
     entries = []
     changed = False
     for c, it in classes.items():
-        key = f"{dev}|{c}"
+        p = it["params"] if it.get("params") is not None else merger.params
+        block = reads_block(p, it["info"].cfa)
+        key = f"{dev}|{KERNELS}|{c}|window{p.window_size_lk}|{'block' if block else 'no block'}"
         if key not in cache:
             n, H, W = it["raw"].shape
             best_rows = _pick(LK_ROWS, lambda r: _time_merge(merger, it, dict(width=W, height=H, lk_strip_rows=r), reps))
-            best_blk = _pick(ACC_BLOCKS, lambda b: _time_merge(merger, it, dict(width=W, height=H, lk_strip_rows=best_rows,
-                                                                                   acc_block_x=b[0], acc_block_y=b[1]), reps))
+            best_blk = ACC_BLOCKS[0]
+            if block:
+                best_blk = _pick(ACC_BLOCKS, lambda b: _time_merge(merger, it, dict(width=W, height=H, lk_strip_rows=best_rows,
+                                                                                       acc_block_x=b[0], acc_block_y=b[1]), reps))
             cache[key] = dict(lk_strip_rows=best_rows, acc_block_x=best_blk[0], acc_block_y=best_blk[1])
             changed = True
         for (W, H) in sorted(sizes[c]):
