@@ -152,14 +152,26 @@ def merge_params():
 _SAMPLE_BURSTS = {}
 
 
-def cpu_reference_run(width, height, threads):
-    """One merge of a sample burst by the reference kernels on the host (FP32, OpenMP); the burst is made once."""
+class ReferenceUnavailable(RuntimeError):
+    """The host build of the reference kernels is not there (it is made from the reference's sources, which are not part of
+    this repository)."""
+
+
+def reference_lib():
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import pipeline as PL
+    try:
+        return PL, PL.StageLib("ref32")
+    except OSError as e:
+        raise ReferenceUnavailable(" ".join(str(e).split())) from e
+
+
+def cpu_reference_run(width, height, threads):
+    """One merge of a sample burst by the reference kernels on the host (FP32, OpenMP); the burst is made once."""
+    PL, lib = reference_lib()
     if (width, height) not in _SAMPLE_BURSTS:
         _SAMPLE_BURSTS[(width, height)] = make_workload_burst(0, "cpu", width, height)
     b = _SAMPLE_BURSTS[(width, height)]
-    lib = PL.StageLib("ref32")
     lib.set_threads(threads)
     t0 = time.perf_counter()
     r = PL.merge_burst(b, merge_params(), lib=lib)
@@ -171,6 +183,11 @@ def cpu_reference_run(width, height, threads):
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    try:
+        reference_lib()
+    except ReferenceUnavailable as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
         return 0
     threads = os.cpu_count() or 1
     w, h = REF_STEP["width"], REF_STEP["height"]
@@ -755,10 +772,13 @@ def run_ours(args):
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
-        px, dt = cpu_reference_run(SAMPLE["width"], SAMPLE["height"], threads)
-        cpu = {"value": px / 1e6 / dt, "unit": UNIT, "cores": threads, "kind": "reference",
-               "sample": f"{WORKLOAD['frames']} frames of {SAMPLE['width']}x{SAMPLE['height']} (same statistics) merged at 2x by the "
-                         f"reference kernels compiled for the host (FP32, OpenMP), {dt:.1f} s wall"}
+        try:
+            px, dt = cpu_reference_run(SAMPLE["width"], SAMPLE["height"], threads)
+            cpu = {"value": px / 1e6 / dt, "unit": UNIT, "cores": threads, "kind": "reference",
+                   "sample": f"{WORKLOAD['frames']} frames of {SAMPLE['width']}x{SAMPLE['height']} (same statistics) merged at 2x by the "
+                             f"reference kernels compiled for the host (FP32, OpenMP), {dt:.1f} s wall"}
+        except ReferenceUnavailable as e:
+            cpu = {"unavailable": str(e)}
     adjoint = None
     if rank == 0 and world == 1 and not args.no_adjoint:
         adjoint = adjoint_ratio(args)
