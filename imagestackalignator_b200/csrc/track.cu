@@ -36,8 +36,10 @@ __device__ __forceinline__ void tile_offset(int tx, int ty, int T, int Wl, int H
     float pcx = (float)(tx * T + T / 2 - Wl / 2), pcy = (float)(ty * T + T / 2 - Hl / 2);
     sx += cf * pcx - sf * pcy - pcx;
     sy += sf * pcx + cf * pcy - pcy;
-    ox = (int)roundf(sx);
-    oy = (int)roundf(sy);
+    // beyond any image, and far enough from the ends of the integers that positions from here do not wrap round to inside it
+    constexpr int LIM = 1 << 28;
+    ox = isa::clampi((int)roundf(sx), -LIM, LIM);
+    oy = isa::clampi((int)roundf(sy), -LIM, LIM);
 }
 
 // Shared-memory layout of k_track, in floats. The template is stored as

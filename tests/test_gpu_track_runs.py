@@ -50,3 +50,41 @@ def test_runs_equal_single_pairs(cuda, T, S):
     for k in range(len(pairs)):
         g, s, a = search([k])
         assert torch.equal(s[0], scores[k]) and torch.equal(a[0], argmin[k]) and torch.equal(g[0], grids[k]), k
+
+
+def test_shifts_beyond_the_integers(cuda):
+    """Pre-shifts that no integer holds, by CTAs and by warps: replicated borders, as for any block far outside."""
+    import torch
+    T, S, n, tcx, tcy = 32, 2, 6, 40, 30
+    W, H = tcx * T + 2 * S, tcy * T + 2 * S
+    rng = np.random.default_rng(8)
+    frames = [torch.from_numpy(rng.uniform(0, 1, (H, W)).astype(np.float32)).cuda() for _ in range(n)]
+    ptrs = torch.tensor([f.data_ptr() for f in frames], device="cuda")
+    pairs = [(a, b) for a in range(n) for b in range(a + 1, n)]
+    tab = (isa.IsaTrackPair * len(pairs))()
+    for k, (a, b) in enumerate(pairs):
+        tab[k].reference, tab[k].to_track, tab[k].grid = a, b, k
+    raw = np.frombuffer(bytes(tab), np.uint8).reshape(len(pairs), -1)
+    far = np.zeros((len(pairs), tcy, tcx, 2), np.float32)
+    odd = (3e9, -3e9, 2147483520.0, -2147483648.0, 1e30, -1e30, np.inf, -np.inf, np.nan)
+    near = far.copy()
+    for k in range(len(pairs)):
+        for i, v in enumerate(odd):
+            far[k, i, (k + i) % 3, i % 2] = v
+            near[k, i, (k + i) % 3, i % 2] = 0.0 if np.isnan(v) else np.clip(v, -1e6, 1e6)
+
+    def search(ks, pre):
+        d = torch.from_numpy(raw[ks].copy()).cuda()
+        g = torch.from_numpy(pre).cuda()
+        am = torch.zeros((len(ks), tcy, tcx), dtype=torch.int32, device="cuda")
+        isa.check(isa.lib().isa_track_level(isa.vp(ptrs), SZ(W * 4), W, H, T, S, tcx, tcy, isa.vp(d), len(ks), isa.vp(g), SZ(tcx * 8),
+                                            SZ(tcx * tcy * 8), ctypes.c_float(0.5), None, isa.vp(am), isa.stream_ptr()))
+        torch.cuda.synchronize()
+        return am
+
+    every = list(range(len(pairs)))
+    assert len(pairs) * tcx * tcy >= 8000  # by warps
+    want = search(every, near)
+    assert torch.equal(search(every, far), want)
+    for k in every:
+        assert torch.equal(search([k], far)[0], want[k]), k
