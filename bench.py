@@ -438,7 +438,7 @@ def uneven_batch(args):
 
     untuned = timed(lambda: run(mergers, streams))
     t0 = time.time()
-    entries = tune.tune(mergers[0], items)
+    entries = tune.tune(mergers[0], items, reps=1, beside=mergers[1:])
     tune_s = time.time() - t0
     for m in mergers:
         m.set_tuning(entries)

@@ -16,6 +16,7 @@ the shapes depend on, so a later run on the same kind of GPU reuses them.
 """
 from __future__ import annotations
 
+import functools
 import json
 import os
 from typing import Dict, List, Optional
@@ -50,18 +51,32 @@ def _device_name() -> str:
     return torch.cuda.get_device_name(torch.cuda.current_device())
 
 
-def _time_merge(merger, item, entry, reps: int) -> float:
+def _time_merge(merger, item, entry, reps: int, beside=()) -> float:
+    """Device time of the burst's merge, by every context of `beside` at the same time."""
     import torch
     from . import isa
-    merger.set_tuning([entry])
-    st = isa.merge_batch([merger], [item])  # warm-up (and a check that the shapes run)
-    if any(st):
-        raise RuntimeError(f"merge failed with tuning {entry}: {st}")
+    mergers = [merger, *beside]
+    for m in mergers:
+        m.set_tuning([entry])
+    bursts = [item] + [dict(item, out=torch.empty_like(item["out"])) for _ in beside]
+    here = torch.cuda.current_stream()
+    streams = [torch.cuda.Stream() for _ in mergers] if beside else [here]
+
+    def run():
+        for s in streams:
+            s.wait_stream(here)
+        st = isa.merge_batch(mergers, bursts, streams)
+        if any(st):
+            raise RuntimeError(f"merge failed with tuning {entry}: {st}")
+        for s in streams:
+            here.wait_stream(s)
+
+    run()  # warm-up (and a check that the shapes run)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     torch.cuda.synchronize()
     e0.record()
     for _ in range(reps):
-        isa.merge_batch([merger], [item])
+        run()
     e1.record()
     torch.cuda.synchronize()
     return e0.elapsed_time(e1) / reps
@@ -75,10 +90,14 @@ def _pick(candidates, cost):
     return candidates[best] if t[best] < (1.0 - MARGIN) * t[0] else candidates[0]
 
 
-def tune(merger, items: List[dict], cache_path: Optional[str] = None, reps: int = 3) -> List[Dict[str, int]]:
+def tune(merger, items: List[dict], cache_path: Optional[str] = None, reps: int = 3, beside=()) -> List[Dict[str, int]]:
     """Tuning entries (isa_ctx_set_tuning dicts) for every frame size of `items`
     (isa.merge_batch burst dicts; `params` gives a burst's merge scale), timed on
-    `merger`'s context and cached in `cache_path` (JSON)."""
+    `merger`'s context and cached in `cache_path` (JSON). `beside`: the other
+    contexts of a batch. A burst alone gains from short strips, which cost more
+    work in all and take it from bursts merged side by side: shapes timed alone
+    made sequential merges 3 % faster and a batch on four contexts 4 % slower,
+    so shapes for a batch are timed on all of its contexts at once."""
     path = cache_path or default_cache_path()
     try:
         with open(path) as f:
@@ -100,18 +119,23 @@ def tune(merger, items: List[dict], cache_path: Optional[str] = None, reps: int 
         p = it["params"] if it.get("params") is not None else merger.params
         block = reads_block(p, it["info"].cfa)
         key = f"{dev}|{KERNELS}|{c}|window{p.window_size_lk}|{'block' if block else 'no block'}"
+        cost = _time_merge
+        if beside:
+            key += f"|{1 + len(beside)} contexts"
+            cost = functools.partial(_time_merge, beside=beside)
         if key not in cache:
             n, H, W = it["raw"].shape
-            best_rows = _pick(LK_ROWS, lambda r: _time_merge(merger, it, dict(width=W, height=H, lk_strip_rows=r), reps))
+            best_rows = _pick(LK_ROWS, lambda r: cost(merger, it, dict(width=W, height=H, lk_strip_rows=r), reps))
             best_blk = ACC_BLOCKS[0]
             if block:
-                best_blk = _pick(ACC_BLOCKS, lambda b: _time_merge(merger, it, dict(width=W, height=H, lk_strip_rows=best_rows,
+                best_blk = _pick(ACC_BLOCKS, lambda b: cost(merger, it, dict(width=W, height=H, lk_strip_rows=best_rows,
                                                                                        acc_block_x=b[0], acc_block_y=b[1]), reps))
             cache[key] = dict(lk_strip_rows=best_rows, acc_block_x=best_blk[0], acc_block_y=best_blk[1])
             changed = True
         for (W, H) in sorted(sizes[c]):
             entries.append(dict(width=W, height=H, **cache[key]))
-    merger.set_tuning([])
+    for m in (merger, *beside):
+        m.set_tuning([])
     if changed:
         os.makedirs(os.path.dirname(path) or ".", exist_ok=True)
         with open(path, "w") as f:

@@ -64,3 +64,16 @@ def test_blocks_are_timed_only_where_they_are_read(timed, tmp_path, params, cfa,
 def test_strip_heights_reach_the_short_strips():
     """Small frames run strips of 8 to 24 rows by the library's own choice."""
     assert {8, 16, 24} <= set(tune.LK_ROWS)
+
+
+def test_contexts_side_by_side_have_entries_of_their_own(timed, tmp_path, monkeypatch):
+    """Shapes of a batch are timed on all its contexts, and kept apart from those of a burst alone."""
+    seen = []
+    monkeypatch.setattr(tune, "_time_merge", lambda merger, item, entry, reps, beside=(): seen.append(len(beside)) or
+                        10.0 + (entry["lk_strip_rows"] == 16 and len(beside)) - 2.0 * (entry["lk_strip_rows"] == 16 and not beside))
+    p, path = P.MergeParams(merge_scale=2.0), str(tmp_path / "t.json")
+    m, others = Merger(p), [Merger(p), Merger(p)]
+    assert tune.tune(m, [item(p)], cache_path=path)[0]["lk_strip_rows"] == 16
+    assert tune.tune(m, [item(p)], cache_path=path, beside=others)[0]["lk_strip_rows"] == 0
+    assert set(seen) == {0, 2} and len(json.loads(open(path).read())) == 2
+    assert all(x.entries == [] for x in [m, *others])
