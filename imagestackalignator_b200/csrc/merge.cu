@@ -140,7 +140,8 @@ __device__ __forceinline__ void cfa_levels(unsigned cfa, const float (&v)[3], fl
 // 512: 8e-3 against 9e-7); SAME: one black level for all channels, a constant instead of a select per tap. The division by
 // s is floor_div_f, exact where the taps' positions are below 2^22 (|v| < 2^22: the frames of isa_ctx_create's limits at
 // scale 8 stay below 2^18).
-// Bound: instruction issue, about 1200 instructions per pixel and frame, mostly address arithmetic and predicated sums.
+// Bound: instruction issue (76 % of its slots), 1300 instructions per pixel and frame, mostly address arithmetic and
+// predicated sums, the ALU pipe at 60 %.
 // 6 x 2000x1500 at 1.5x: 1.87 ms, from 5.4 ms with per-tap divisions, indexed channels and normalisation.
 template <int KC, bool SAME>
 __global__ void __launch_bounds__(256, 3) k_accumulate(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
@@ -423,7 +424,8 @@ __device__ __forceinline__ void loss_sum(double lsum, double* loss)
 // ((raw - black) - white out) (h / white), a tap costs no division (black comes off the sample by itself: rounded into one
 // number with white out it would cost the residual its last digits in dark areas); the channel's factors come per row and
 // column parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
-// Bound: instruction issue and the mask-certainty atomics (one per tap and frame). 6 x 2000x1500 at 1.5x: 3.1 ms, from
+// Bound: the mask-certainty atomics (one per tap and frame) and issue (56 % of its slots, 1600 instructions per pixel and
+// frame). 6 x 2000x1500 at 1.5x: 3.1 ms, from
 // 8.0 ms with a division and branches on the channel per tap.
 template <int KC>
 __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,

@@ -36,8 +36,9 @@
 // weights so large that their sums could overflow) take a per-tap path with
 // the reference's clamps, out of line.
 //
-// Bound: instruction issue and instruction fetch, about 290 instructions per
-// pixel and frame at an IPC near 2.7. Code size decides as much as the count:
+// Bound: instruction issue and instruction fetch, 316 instructions per pixel
+// and frame over 8 frames (the pixel's own set-up among them) at an IPC of 2.5,
+// the ALU pipe at 50 %. Code size decides as much as the count:
 // the frame loop is one body per Y mod 4 (uniform in a CTA, and the rows of a
 // 32-row band run one Y mod 4 after another) with a 35-instruction section
 // per X mod 4. One body per (X mod 4, Y mod 4) pair inside a CTA took 157 ms
@@ -414,8 +415,9 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
 // parameter, uniform in a CTA; the column pattern is a select per lane.
 // Black comes off each sample (see k_accumulate); SAME: one level for all
 // channels, a constant instead of four selected ones (and their spills).
-// Bound: instruction issue, 100 additions and multiply-adds and about as many
-// selects and loads per pixel and frame. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
+// Bound: issue and the loads' latency, 386 instructions per pixel and frame over
+// 8 frames (100 additions and multiply-adds, about as many selects and loads) at
+// an IPC of 2.2, 26 of 64 warps. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
 // with its clamps, divisions and indexed channels; one 3010x2006 frame by
 // itself 0.22 ms, from 0.72 ms. CTAs of 512 threads: 2.9 ms and 0.24 ms; at 80
 // registers (24 warps per SM) 3.0 ms.

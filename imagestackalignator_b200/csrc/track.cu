@@ -309,7 +309,7 @@ cudaError_t launch_track_ts(const float* const* frames, size_t pitch, int Wl, in
 // registers, so the chain pair table -> pre-shift -> frame table -> tile loads
 // is off the critical path.
 // Bound: the FMA pipe (2 lane operations per template pixel and shift), busy
-// about 60 %; 12 warps per SM (S = 2, 15 KB of shared memory each; at S = 5 and 6,
+// 59 %; 12 warps per SM (S = 2, 15 KB of shared memory each; at S = 5 and 6,
 // 19 and 21 KB, 8) leave the chains of staging and minimum search partly exposed. All 190 pairs of 20 x 6016x4000:
 // tile alignment (four levels and solves) 29.1 -> 23.0 ms.
 template <int T, int S>
