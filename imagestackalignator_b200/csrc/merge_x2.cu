@@ -198,7 +198,7 @@ __device__ __forceinline__ float tap_weights(float k0, float k1, float k2, float
 
 // One frame's sums of a pixel tap by tap at scale S (1 or 2), with the crop clamps and mirrored flow of the reference.
 // Scale 1: a is normalised; scale 2: a holds the sums of w cert raw.
-template <int S>
+template <int S, bool SAME>
 __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
 {
     constexpr int SH = S - 1;
@@ -241,7 +241,8 @@ __device__ __noinline__ Sums frame_per_tap(const X2Args& A, int f, int x, int y)
             }
             const float wc = __fmul_rn(w[py + 2][d], cert);
             float v = (float)__ldg(rr + qx[d]);
-            if constexpr (S == 1) v = __fmaf_rn(v, A.lv.scale, c == 0 ? A.lv.nblack[0] : (c == 1 ? A.lv.nblack[1] : A.lv.nblack[2]));
+            if constexpr (S == 1)
+                v = __fmaf_rn(v, A.lv.scale, SAME ? A.lv.nblack[0] : (c == 0 ? A.lv.nblack[0] : (c == 1 ? A.lv.nblack[1] : A.lv.nblack[2])));
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 if (k == c) { s.w[k] = __fadd_rn(s.w[k], wc); s.a[k] = __fmaf_rn(wc, v, s.a[k]); }
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
                 default: f = frames_x2<3, SANE>(A, f, x, y, w, interior, a, ws); break;
                 }
                 if (f >= A.nframes) break;
-                const Sums s = frame_per_tap<2>(A, f, x, y);
+                const Sums s = frame_per_tap<2, true>(A, f, x, y);
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     a[c] += (s.a[c] - A.black.v[c] * s.w[c]) * A.rwhite.v[c];
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(X1_NT, X1_CTAS) k_accumulate_x1(const __grid_c
         if ((Y & 1) == 0) f = frames_x1<0, SANE, SAME>(A, f, X, Y, w, interior, a, ws);  // the same for the whole CTA
         else f = frames_x1<1, SANE, SAME>(A, f, X, Y, w, interior, a, ws);
         if (f >= A.nframes) break;
-        const Sums s = frame_per_tap<1>(A, f, x, y);
+        const Sums s = frame_per_tap<1, SAME>(A, f, x, y);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             a[c] += s.a[c];
