@@ -427,7 +427,7 @@ __device__ __forceinline__ void loss_sum(double lsum, double* loss)
 // Bound: the mask-certainty atomics (one per tap and frame) and issue (56 % of its slots, 1600 instructions per pixel and
 // frame). 6 x 2000x1500 at 1.5x: 3.1 ms, from
 // 8.0 ms with a division and branches on the channel per tap.
-template <int KC>
+template <int KC, bool SAME>
 __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
                                                        size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* __restrict__ kparam,
                                                        size_t kp_pitch, F3 white, F3 black, const float* __restrict__ out, size_t out_pitch,
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, uns
                     for (int px = 0; px < 5; px++) {
                         const int t = py * 5 + px;
                         const bool odd = qx[px] & 1;
-                        const float r = (((float)__ldg(rr + qx[px]) - (odd ? bo : be)) - (odd ? oo : oe)) * (odd ? ho : he);
+                        const float r = (((float)__ldg(rr + qx[px]) - (SAME ? black.v[0] : (odd ? bo : be))) - (odd ? oo : oe)) * (odd ? ho : he);
                         float cert = 1.f;
                         if (fr.mask) {
                             const size_t at = mrow + 4u * (unsigned)(ux[px] + (odd ? co : ce));
@@ -802,12 +802,13 @@ cudaError_t isa_launch_accumulate_bwd(const isa_accum_geom& g, unsigned cfa, con
 {
     F3 wh, bl;
     for (int c = 0; c < 3; c++) { wh.v[c] = white[c]; bl.v[c] = black[c]; }
+    const bool same = black[0] == black[1] && black[0] == black[2];
     dim3 b(32, 8), grd = grid2(g.Wo, g.Ho, b);
     if (g.bilinear)
         k_accumulate_bwd_bil<4><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out,
                                                    out_pitch, wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss, gflow);
     else
-        k_accumulate_bwd<4><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out, out_pitch,
+        (same ? k_accumulate_bwd<4, true> : k_accumulate_bwd<4, false>)<<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out, out_pitch,
                                                wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss);
     return cudaGetLastError();
 }

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
 // channels, a constant instead of four selected ones (and their spills).
 // Bound: issue and the loads' latency, 386 instructions per pixel and frame over
 // 8 frames (100 additions and multiply-adds, about as many selects and loads) at
-// an IPC of 2.2, 26 of 64 warps. 12 x 4000x3000: 2.8 ms, from 15.9 ms tap by tap
+// an IPC of 2.2, 26 of 64 warps. 12 x 4000x3000: 2.74 ms, from 15.9 ms tap by tap
 // with its clamps, divisions and indexed channels; one 3010x2006 frame by
 // itself 0.22 ms, from 0.72 ms. CTAs of 512 threads: 2.9 ms and 0.24 ms; at 80
 // registers (24 warps per SM) 3.0 ms.
