@@ -425,8 +425,7 @@ __device__ __forceinline__ void loss_sum(double lsum, double* loss)
 // number with white out it would cost the residual its last digits in dark areas); the channel's factors come per row and
 // column parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
 // Bound: the mask-certainty atomics (one per tap and frame) and issue (56 % of its slots, 1600 instructions per pixel and
-// frame). 6 x 2000x1500 at 1.5x: 3.1 ms, from
-// 8.0 ms with a division and branches on the channel per tap.
+// frame); SAME as in k_accumulate. 6 x 2000x1500 at 1.5x: 3.1 ms, from 8.0 ms with a division and branches on the channel per tap.
 template <int KC, bool SAME>
 __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,
                                                        size_t raw_pitch, size_t flow_pitch, size_t mask_pitch, const float* __restrict__ kparam,
@@ -808,8 +807,9 @@ cudaError_t isa_launch_accumulate_bwd(const isa_accum_geom& g, unsigned cfa, con
         k_accumulate_bwd_bil<4><<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out,
                                                    out_pitch, wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss, gflow);
     else
-        (same ? k_accumulate_bwd<4, true> : k_accumulate_bwd<4, false>)<<<grd, b, 0, st>>>(g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out, out_pitch,
-                                               wsum, ws_pitch, target, tg_pitch, weight, wt_pitch, gkp, gmask, gmask_stride, loss);
+        (same ? k_accumulate_bwd<4, true> : k_accumulate_bwd<4, false>)<<<grd, b, 0, st>>>(
+            g, cfa, frames, nframes, raw_pitch, flow_pitch, mask_pitch, kparam, kparam_pitch, wh, bl, out, out_pitch, wsum, ws_pitch, target, tg_pitch,
+            weight, wt_pitch, gkp, gmask, gmask_stride, loss);
     return cudaGetLastError();
 }
 

@@ -111,8 +111,8 @@ def test_large_weights_stay_finite(cuda, scale, kc):
     assert (w > 0).all() and (a / w).max() <= 1.0 + 1e-5 and (a / w).min() >= -512.0 / 15871.0 - 1e-5
 
 
-@pytest.mark.parametrize("scale", [1.5, 3.0])
-def test_gradient_keeps_the_last_digits_of_dark_frames(cuda, scale):
+@pytest.mark.parametrize("scale,over", [(1.5, (0, 0, 0)), (3.0, (0, 0, 0)), (1.5, (1, 0, 2))])
+def test_gradient_keeps_the_last_digits_of_dark_frames(cuda, scale, over):
     """Equal frames of 1 .. 20 over black: no motion, full certainty, so raising the samples and black by 49152 changes
     nothing the gradient depends on. The two gradients differ by the order of the FP32 atomic sums alone: a term per
     weighted pixel and tap, 200 in all, so 200 * 2^-24 = 1.2e-5 of the terms' magnitudes; a few pixels are weighted, so that
@@ -128,7 +128,7 @@ def test_gradient_keeps_the_last_digits_of_dark_frames(cuda, scale):
         info = isa.IsaRawInfo()
         info.width, info.height = W, H
         info.cfa[:] = (0, 1, 1, 2)
-        info.black[:] = (float(lift),) * 3
+        info.black[:] = tuple(float(lift + o) for o in over)
         info.white[:] = (15871.0,) * 3
         info.camera_white[:] = (1.0,) * 3
         info.noise_alpha, info.noise_beta = 1e-3, 8e-6
