@@ -424,7 +424,7 @@ __device__ __forceinline__ void loss_sum(double lsum, double* loss)
 // ((raw - black) - white out) (h / white), a tap costs no division (black comes off the sample by itself: rounded into one
 // number with white out it would cost the residual its last digits in dark areas); the channel's factors come per row and
 // column parity; dL/dw is kept for the 13 distinct weights (dq/dk is the same for a tap and its opposite).
-// Bound: the mask-certainty atomics (one per tap and frame) and issue (56 % of its slots, 1600 instructions per pixel and
+// Bound: the mask-certainty atomics (one per tap and frame) and issue (56 % of its slots, 1550 instructions per pixel and
 // frame); SAME as in k_accumulate. 6 x 2000x1500 at 1.5x: 3.1 ms, from 8.0 ms with a division and branches on the channel per tap.
 template <int KC, bool SAME>
 __global__ void __launch_bounds__(256, 3) k_accumulate_bwd(isa_accum_geom g, unsigned cfa, const isa_frame_in* __restrict__ frames, int nframes,

@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(X2_NT, X2_CTAS) k_accumulate_x2(const __grid_c
 // parameter, uniform in a CTA; the column pattern is a select per lane.
 // Black comes off each sample (see k_accumulate); SAME: one level for all
 // channels, a constant instead of four selected ones (and their spills).
-// Bound: issue and the loads' latency, 386 instructions per pixel and frame over
+// Bound: issue and the loads' latency, 385 instructions per pixel and frame over
 // 8 frames (100 additions and multiply-adds, about as many selects and loads) at
 // an IPC of 2.2, 26 of 64 warps. 12 x 4000x3000: 2.74 ms, from 15.9 ms tap by tap
 // with its clamps, divisions and indexed channels; one 3010x2006 frame by
